@@ -38,11 +38,12 @@ WORKLOAD = "procedural-room-1M-tris-1080p-4spp-restirdi32-atrous5"
 CFG = dict(width=1920, height=1080, spp=4, max_bounces=5, di_candidates=32, di_neighbors=5, di_radius=30,
            m_cap_factor=20, atrous_iterations=5, scene_seed=0x5EED0002, triangles=1_000_000, emitters=4096,
            box_half=20.0, eye=(0.0, 4.0, 34.0), center=(0.0, -3.0, 0.0))
-# Algorithmic bytes (per unit): a ray record 32 B in + 16 B hit out, a BVH2
-# node (two child boxes) 64 B, a triangle (3 vertices) 36 B.
-# A node of the 4-wide tree (the wide traversal variants) holds four child
-# boxes: 128 B (rr_pathtracer_variant_width).
-RAY_BYTES, NODE_BYTES, TRI_BYTES = 48, 64, 36
+# Algorithmic bytes (per unit): a ray record 32 B in + 16 B hit out, a child
+# box with its reference 16 B (quantized trees; rr_pathtracer_variant_width
+# boxes a node) or 32 B (variant 7, full precision), a triangle (3 vertices)
+# 36 B.
+RAY_BYTES, CHILD_BYTES, TRI_BYTES = 48, 16, 36
+FULL_PRECISION_VARIANT = 7
 
 
 def parse():
@@ -545,8 +546,8 @@ def run_ours(args, ws, rank, local):
 
     # roofline of the dominant kernel (BVH traversal of extension rays)
     peak, peak_kind = load_peaks()
-    node_bytes = {k: NODE_BYTES * rr.lib().rr_pathtracer_variant_width(tuned[k + "_variant"]) // 2
-                  for k in ("extend", "shadow")}
+    node_bytes = {k: CHILD_BYTES * (2 if tuned[k + "_variant"] == FULL_PRECISION_VARIANT else 1) *
+                  rr.lib().rr_pathtracer_variant_width(tuned[k + "_variant"]) for k in ("extend", "shadow")}
     ext_bytes = (counted["extension_rays"] * RAY_BYTES + counted["extension_nodes"] * node_bytes["extend"] +
                  counted["extension_tris"] * TRI_BYTES)
     ext_ms = pt_stage["extend"]

@@ -142,18 +142,17 @@ typedef struct rr_pt_stats {
 rr_status rr_pathtracer_stats(rr_ctx* ctx, rr_pt_stats* out, int reset_times);
 
 /* Traversal kernel variants (no reference counterpart; the reference uses
- * hardware ray queries): variant = tree x stack x occupancy target; every
- * warp traces 32 consecutive queue entries to completion.
- *   0: binary tree, stack in local memory, the compiler's register count
- *      (default);
- *   1: as 0 with a register budget for 5 blocks of 256 threads per SM;
- *   2: as 0 with the bottom 8 stack entries in shared memory;
- *   5: as 2 with a budget for 5 blocks;
- *   3, 4, 6: the 4-wide tree (rr_pathtracer_variant_width), stack in local
- *      memory / bottom 8 entries in shared memory / as 4 with a budget for 3
- *      blocks;
- *   7: binary tree with leaves postponed until every lane of the warp holds
- *      one, budget for 4 blocks.
+ * hardware ray queries): variant = tree x stack x occupancy target (blocks
+ * of 256 threads per SM). 0 to 6 walk the scene's trees with boxes quantized
+ * to a 15-bit grid (a box only grows, so hits are the same), a warp's lanes
+ * in step, idle lanes taking new rays:
+ *   0, 1, 2, 5: binary tree: bottom 8 stack entries in shared memory; local
+ *      stack, 5 blocks; local stack; bottom 12 in shared memory, 5 blocks;
+ *   3, 4, 6: 4-wide tree (rr_pathtracer_variant_width): local stack; bottom
+ *      12 entries in shared memory (4, the default); bottom 8, 5 blocks;
+ *   7: binary tree in full precision, one thread per ray. Scenes whose boxes
+ *      the grid would grow too much (a few triangles far from all others)
+ *      use it whatever the variant.
  * Results are identical for every variant; only speed differs. */
 #define RR_PT_VARIANT_COUNT 8
 rr_status rr_pathtracer_set_variants(rr_ctx* ctx, int extend_variant, int shadow_variant);

@@ -13,6 +13,8 @@
 
 #include "rr_bvh.h"
 
+#include <vector_functions.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -190,6 +192,109 @@ struct Wide4 {
     }
 };
 
+// A child's reference as the quantized nodes hold it: an inner node's index,
+// or a leaf's first triangle and count (1 to 15) under the sign bit.
+bool quant_ref(int32_t ref, int32_t count, uint32_t& out) {
+    if (ref >= 0) { out = uint32_t(ref); return true; }
+    const uint32_t first = uint32_t(~ref);
+    if (first >= (1u << 27) || count < 0 || count > 15) return false;
+    out = 0x80000000u | (first << 4) | uint32_t(count);
+    return true;
+}
+
+// The quantized forms of both trees: every box plane goes outwards to a plane
+// of a 15-bit grid over the scene's bounds, so a box only grows. Refused (the
+// traversals then read the trees in full precision) where the boxes would
+// grow by more than kQuantGrowth in surface area, summed over the tree (a
+// few triangles far from all others stretch the grid), and where a leaf or a
+// coordinate does not fit the format. Measured on the 1M-triangle room (960 x
+// 540, 4 spp) with one mesh moved away, extension / shadow ms quantized
+// against full precision (4.7 / 3.4): growth 1.003 2.6 / 1.6, 1.010 2.7 / 1.7,
+// 1.036 3.4 / 2.1, 1.094 5.3 / 3.5, 1.2 10.0 / 7.3. The 10M-triangle instanced
+// scenes grow by 1.006 and 1.008.
+constexpr double kQuantGrowth = 1.06;
+
+bool quantize_trees(BvhBuild& out) {
+    const size_t n = out.nodes.size() / 4, n4 = out.nodes4.size() / 8;
+    if (n >= 0x7ffffff0u) return false;
+    // lower and upper plane of one child on one axis
+    auto planes = [&](size_t g, int child, int a, float& l, float& h) {
+        const float4* q = &out.nodes[g * 4];
+        const float4& xy = q[child];
+        const float4& z = q[2];
+        if (a == 0) { l = xy.x; h = xy.y; }
+        else if (a == 1) { l = xy.z; h = xy.w; }
+        else { l = child ? z.z : z.x; h = child ? z.w : z.y; }
+    };
+    double first[3], cell[3];   // plane 0 and the grid's step, as the kernels see them
+    for (int a = 0; a < 3; ++a) {
+        float l0, h0, l1, h1;
+        planes(0, 0, a, l0, h0);
+        planes(0, 1, a, l1, h1);
+        const double lo = std::min(l0, l1), hi = std::max(h0, h1);
+        const double big = std::max(std::fabs(lo), std::fabs(hi));
+        if (!(big < 1e12)) return false;
+        // no step finer than the coordinates' own spacing
+        const double c = std::max((hi - lo) / 32760.0, std::max(big, 1e-12) * 1.2e-7);
+        out.qscale[a] = std::nextafter(float(c * 256.0), INFINITY);
+        cell[a] = double(out.qscale[a]) / 256.0;
+        out.qbase[a] = float(lo - 2.0 * cell[a] - 128.0 * double(out.qscale[a]));
+        first[a] = double(out.qbase[a]) + 128.0 * double(out.qscale[a]);
+    }
+    auto pack = [&](int a, float l, float h, uint32_t& w, double& extent) {
+        const double ql = std::floor((double(l) - first[a]) / cell[a] - 1e-6);
+        const double qh = std::ceil((double(h) - first[a]) / cell[a] + 1e-6);
+        if (!(ql >= 0.0 && qh <= 32767.0 && ql <= qh)) return false;
+        w = uint32_t(ql) | (uint32_t(qh) << 16);
+        extent = (qh - ql) * cell[a];
+        return true;
+    };
+    auto area = [](const double* e) { return e[0] * e[1] + e[1] * e[2] + e[2] * e[0]; };
+    double full = 0.0, grown = 0.0;
+    out.qnodes.resize(n * 2);
+    for (size_t g = 0; g < n; ++g) {
+        const float4& d = out.nodes[g * 4 + 3];
+        int32_t ref[2], cnt[2];
+        std::memcpy(ref, &d.x, 8);
+        std::memcpy(cnt, &d.z, 8);
+        for (int c = 0; c < 2; ++c) {
+            double e[3], eq[3];
+            uint32_t w[3], r;
+            for (int a = 0; a < 3; ++a) {
+                float l, h;
+                planes(g, c, a, l, h);
+                if (!pack(a, l, h, w[a], eq[a])) return false;
+                e[a] = double(h) - double(l);
+            }
+            full += area(e);
+            grown += area(eq);
+            if (!quant_ref(ref[c], cnt[c], r)) return false;
+            out.qnodes[g * 2 + c] = make_uint4(w[0], w[1], w[2], r);
+        }
+    }
+    if (!(grown <= kQuantGrowth * full)) return false;
+    out.qnodes4.resize(n4 * 4);
+    for (size_t g = 0; g < n4; ++g) {
+        const float* f = &out.nodes4[g * 8].x;
+        for (int k = 0; k < 4; ++k) {
+            uint32_t w[3], r;
+            double extent;
+            if (!(f[k] < 1e29f)) {   // an unused slot: lower plane above the upper one, an empty leaf
+                out.qnodes4[g * 4 + k] = make_uint4(32767u, 32767u, 32767u, 0x80000000u);
+                continue;
+            }
+            int32_t ref, cnt;
+            std::memcpy(&ref, f + 24 + k, 4);
+            std::memcpy(&cnt, f + 28 + k, 4);
+            for (int a = 0; a < 3; ++a)
+                if (!pack(a, f[a * 8 + k], f[a * 8 + 4 + k], w[a], extent)) return false;
+            if (!quant_ref(ref, cnt, r)) return false;
+            out.qnodes4[g * 4 + k] = make_uint4(w[0], w[1], w[2], r);
+        }
+    }
+    return true;
+}
+
 } // namespace
 
 BvhBuild build_bvh(const std::vector<float>& tri_world, int /*threads*/) {
@@ -237,6 +342,7 @@ BvhBuild build_bvh(const std::vector<float>& tri_world, int /*threads*/) {
         out.nodes.push_back(mk4(lo0, hi0, lo1, hi1));
         out.nodes.push_back(mk4(lo2, hi2, lo2, hi2));
         out.nodes.push_back(mk4(i2f(~int32_t(0)), i2f(~int32_t(0)), i2f(int32_t(r.count)), i2f(0)));
+        if (!quantize_trees(out)) { out.qnodes.clear(); out.qnodes4.clear(); }
         return out;
     }
     // iterative DFS to assign GPU indices
@@ -262,6 +368,7 @@ BvhBuild build_bvh(const std::vector<float>& tri_world, int /*threads*/) {
         out.nodes[g * 4 + 2] = mk4(c0.box.lo[2], c0.box.hi[2], c1.box.lo[2], c1.box.hi[2]);
         out.nodes[g * 4 + 3] = mk4(i2f(r0), i2f(r1), i2f(k0), i2f(k1));
     }
+    if (!quantize_trees(out)) { out.qnodes.clear(); out.qnodes4.clear(); }
     return out;
 }
 

@@ -949,8 +949,8 @@ extern "C" rr_status rr_guided_pathtracer_execute(rr_ctx* ctx, const rr_scene* s
                                                                                        q.ray_c[0], C);
         RR_CHECK_LAUNCH(ctx);
     }
-    QueueKernel ext_k = extend_variant<false>(ctx->extend_variant);
-    ShadowKernel sh_k = shadow_variant<false>(ctx->shadow_variant);
+    QueueKernel ext_k = extend_variant<false>(variant_for(scene->dev, ctx->extend_variant));
+    ShadowKernel sh_k = shadow_variant<false>(variant_for(scene->dev, ctx->shadow_variant));
     const int g_ext = persistent_grid(ctx, reinterpret_cast<const void*>(ext_k));
     const int g_sh = persistent_grid(ctx, reinterpret_cast<const void*>(sh_k));
     const bool emitters = (p->flags & RR_PT_FLAG_EMITTERS) != 0;
@@ -1276,8 +1276,8 @@ static rr_status enqueue_guided_batch(rr_ctx* ctx, rr_batch* B, rr_guide* const*
         RR_CHECK_LAUNCH(ctx);
         launches += 1;
     }
-    BatchQueueKernel ext_k = extend_batch_variant<false>(ctx->extend_variant);
-    BatchShadowKernel sh_k = shadow_batch_variant<false>(ctx->shadow_variant);
+    BatchQueueKernel ext_k = extend_batch_variant<false>(B->quantized ? ctx->extend_variant : kVariantFull);
+    BatchShadowKernel sh_k = shadow_batch_variant<false>(B->quantized ? ctx->shadow_variant : kVariantFull);
     const int g_ext = persistent_grid(ctx, reinterpret_cast<const void*>(ext_k));
     const int g_sh = persistent_grid(ctx, reinterpret_cast<const void*>(sh_k));
     auto shade_k = mlp ? guided_shade_kernel<true, true> : guided_shade_kernel<false, true>;

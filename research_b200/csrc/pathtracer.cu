@@ -386,8 +386,9 @@ extern "C" rr_status rr_pathtracer_execute(rr_ctx* ctx, const rr_scene* scene,
     }
     const bool count = (p->flags & RR_PT_FLAG_COUNT_TRAVERSAL) != 0;
     const bool timed = (p->flags & RR_PT_FLAG_TIME_STAGES) != 0;
-    QueueKernel ext_k = count ? extend_variant<true>(ctx->extend_variant) : extend_variant<false>(ctx->extend_variant);
-    ShadowKernel sh_k = count ? shadow_variant<true>(ctx->shadow_variant) : shadow_variant<false>(ctx->shadow_variant);
+    const int ev = variant_for(scene->dev, ctx->extend_variant), sv = variant_for(scene->dev, ctx->shadow_variant);
+    QueueKernel ext_k = count ? extend_variant<true>(ev) : extend_variant<false>(ev);
+    ShadowKernel sh_k = count ? shadow_variant<true>(sv) : shadow_variant<false>(sv);
     const int g_ext = persistent_grid(ctx, reinterpret_cast<const void*>(ext_k));
     const int g_sh = persistent_grid(ctx, reinterpret_cast<const void*>(sh_k));
     const bool emitters = (p->flags & RR_PT_FLAG_EMITTERS) != 0;
@@ -552,10 +553,10 @@ rr_status enqueue_batch(rr_ctx* ctx, rr_batch* B, uint32_t total_tiles, size_t n
         rr_status st0 = t0.commit();
         if (st0 != RR_OK) return st0;
     }
-    BatchQueueKernel ext_k = count ? extend_batch_variant<true>(ctx->extend_variant)
-                                   : extend_batch_variant<false>(ctx->extend_variant);
-    BatchShadowKernel sh_k = count ? shadow_batch_variant<true>(ctx->shadow_variant)
-                                   : shadow_batch_variant<false>(ctx->shadow_variant);
+    const int ev = B->quantized ? ctx->extend_variant : kVariantFull;
+    const int sv = B->quantized ? ctx->shadow_variant : kVariantFull;
+    BatchQueueKernel ext_k = count ? extend_batch_variant<true>(ev) : extend_batch_variant<false>(ev);
+    BatchShadowKernel sh_k = count ? shadow_batch_variant<true>(sv) : shadow_batch_variant<false>(sv);
     const int g_ext = persistent_grid(ctx, reinterpret_cast<const void*>(ext_k));
     const int g_sh = persistent_grid(ctx, reinterpret_cast<const void*>(sh_k));
     const int g_shade = std::min<int>(persistent_grid(ctx, reinterpret_cast<const void*>(shade_kernel<true>)),
@@ -635,7 +636,10 @@ extern "C" rr_status rr_batch_create(rr_ctx* ctx, const rr_scene* const* scenes,
     B->scenes.assign(scenes, scenes + count);
     auto fail = [&](rr_status s) { rr_batch_destroy(B); return s; };
     std::vector<rr::DevScene> table(count);
-    for (uint32_t i = 0; i < count; ++i) table[i] = scenes[i]->dev;
+    for (uint32_t i = 0; i < count; ++i) {
+        table[i] = scenes[i]->dev;
+        B->quantized = B->quantized && table[i].qnodes4;
+    }
     B->entries_bytes = (sizeof(rr::BatchEntry) * count + 15) & ~size_t(15);
     B->call_bytes = B->entries_bytes + sizeof(void*) * count;
     cudaError_t e;

@@ -572,17 +572,19 @@ rr_status gi_initial_wavefront(rr_ctx* ctx, const rr_scene* scene, const GpuCame
     const int g_begin = std::min<int>(persistent_grid(ctx, reinterpret_cast<const void*>(giw_begin_kernel)), cap);
     giw_begin_kernel<<<g_begin, kBlock, 0, stream>>>(S, L, I, V);
     RR_CHECK_LAUNCH(ctx);
-    const int g_ext = persistent_grid(ctx, reinterpret_cast<const void*>(wave_extend_kernel));
-    const int g_sh = persistent_grid(ctx, reinterpret_cast<const void*>(wave_shadow_kernel));
+    const WaveExtendKernel ext_k = wave_extend(S);
+    const WaveShadowKernel sh_k = wave_shadow(S);
+    const int g_ext = persistent_grid(ctx, reinterpret_cast<const void*>(ext_k));
+    const int g_sh = persistent_grid(ctx, reinterpret_cast<const void*>(sh_k));
     const int g_shade = std::min<int>(persistent_grid(ctx, reinterpret_cast<const void*>(giw_shade_kernel)), cap);
     const int g_adv = std::min<int>(persistent_grid(ctx, reinterpret_cast<const void*>(giw_advance_kernel)), cap);
     for (uint32_t k = 0; k < steps; ++k) {
         uint32_t* c0 = cnt + size_t(k) * kWaveWords;
-        wave_extend_kernel<<<g_ext, kBlock, 0, stream>>>(S, V.qa[k & 1], V.qb[k & 1], V.hits, c0, L.ray_bias);
+        ext_k<<<g_ext, kBlock, 0, stream>>>(S, V.qa[k & 1], V.qb[k & 1], V.hits, c0, L.ray_bias);
         RR_CHECK_LAUNCH(ctx);
         giw_shade_kernel<<<g_shade, kBlock, 0, stream>>>(S, L, V, k);
         RR_CHECK_LAUNCH(ctx);
-        wave_shadow_kernel<<<g_sh, kBlock, 0, stream>>>(S, V.sa, V.sb, V.sc, V.rad, c0, L.ray_bias);
+        sh_k<<<g_sh, kBlock, 0, stream>>>(S, V.sa, V.sb, V.sc, V.rad, c0, L.ray_bias);
         RR_CHECK_LAUNCH(ctx);
         giw_advance_kernel<<<g_adv, kBlock, 0, stream>>>(S, L, I, V, k);
         RR_CHECK_LAUNCH(ctx);

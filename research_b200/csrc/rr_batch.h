@@ -15,6 +15,7 @@ struct rr_batch {
     rr_ctx* ctx = nullptr;
     std::vector<const rr_scene*> scenes;
     rr::DevScene* d_table = nullptr;       // per scene, uploaded once
+    bool quantized = true;                 // every scene has the quantized trees
     unsigned char* d_call = nullptr;       // per call: BatchEntry[count], then float4*[count]
     unsigned char* h_call[2] = {nullptr, nullptr};  // pinned staging of d_call, alternating
     cudaEvent_t staged[2] = {nullptr, nullptr};     // the copy out of h_call[k] has completed

@@ -28,6 +28,9 @@ struct DevScene {
     const float4* nodes;
     const float4* tris;
     const float4* nodes4;     // the same tree 4-wide (see trace_step4)
+    const uint4* qnodes;      // both trees with quantized boxes (see QuantRay), or null
+    const uint4* qnodes4;
+    float3 qbase, qscale;     // grid plane q of an axis: qbase + (128 + q / 256) * qscale
     const float4* vertices;   // GpuVertex as 3 float4
     const uint32_t* indices;
     const uint4* meshes;      // GpuMesh as 2 uint4
@@ -175,19 +178,16 @@ struct TraceWork {
     uint32_t tris = 0;
 };
 
-// Traversal state of one ray between node steps. node < 0: no inner node
-// left, only the postponed leaf (pend_count > 0) to intersect.
+// Traversal state of one ray between node steps.
 struct TravState {
     int node;
     int sp;
     bool found;
     uint32_t visits;
-    int pend_first, pend_count;
 };
 
 RR_D void trav_begin(TravState& st, HitRec& hit, float tmax) {
     st.node = 0; st.sp = 0; st.found = false; st.visits = 0;
-    st.pend_first = 0; st.pend_count = 0;
     hit.t = tmax; hit.key = kNoIndex;
 }
 
@@ -224,23 +224,26 @@ RR_D bool leaf_tris(const DevScene& s, const Ray& r, float tmin, HitRec& hit, Tr
 // compete with node and triangle fetches for L1 lines.
 // N entries: kStackSize for the binary tree (one push per level, at most 60
 // levels), kStackSize4 for the 4-wide tree (at most three pushes per level).
+// Entry: int2, or int where the near distance is not needed (any hit).
 constexpr int kStackSize4 = 192;
-template <int N = kStackSize>
+template <int N = kStackSize, class E = int2>
 struct LocalStackN {
-    int2 e[N];
-    RR_D void put(int i, int2 v) { e[i] = v; }
-    RR_D int2 get(int i) const { return e[i]; }
+    using Entry = E;
+    E e[N];
+    RR_D void put(int i, E v) { e[i] = v; }
+    RR_D E get(int i) const { return e[i]; }
 };
 using LocalStack = LocalStackN<kStackSize>;
-template <int S, int Threads, int N = kStackSize>
+template <int S, int Threads, int N = kStackSize, class E = int2>
 struct SplitStack {
-    int2* col;
-    int2 e[N - S];
-    RR_D void put(int i, int2 v) {
+    using Entry = E;
+    E* col;
+    E e[N - S];
+    RR_D void put(int i, E v) {
         if (i < S) col[i * Threads] = v;
         else e[i - S] = v;
     }
-    RR_D int2 get(int i) const { return i < S ? col[i * Threads] : e[i - S]; }
+    RR_D E get(int i) const { return i < S ? col[i * Threads] : e[i - S]; }
 };
 
 // Pops the next stacked node not beyond the current hit; false when none is left.
@@ -262,25 +265,9 @@ RR_D bool pop_node(TravState& st, const Stack& stack, const HitRec& hit) {
 // fewer node visits on the 1M-triangle room). An any-hit ray only reports
 // whether a triangle lies in [tmin, tmax], which no visiting order changes.
 // Returns true once the traversal is finished (stack empty, or any hit).
-// Postpone: a lane keeps its first leaf child for later and goes on with
-// inner nodes; the step intersects the kept leaf once every lane of the warp
-// still traversing holds one (or the lane has no inner node left), so the
-// warp runs its leaves' triangle loops side by side instead of one lane's
-// at a time (Aila and Laine 2009). Culling meanwhile uses the hit found so
-// far, which only visits more, and the kept (t, key) minimum does not depend
-// on the order, so the result is the same.
-template <bool AnyHit, bool Count, bool Postpone = false, class Stack>
+template <bool AnyHit, bool Count, class Stack>
 RR_D bool trace_step(const DevScene& s, const Ray& r, float tmin, HitRec& hit, TravState& st,
                      Stack& stack, TraceWork* work) {
-    if constexpr (Postpone) {
-        const bool all_hold = __all_sync(__activemask(), st.pend_count > 0);
-        if (st.pend_count > 0 && (st.node < 0 || all_hold)) {
-            if (leaf_tris<AnyHit, Count>(s, r, tmin, hit, st, st.pend_first, st.pend_count, work)) return true;
-            st.pend_count = 0;
-            if (st.node >= 0) return false;
-            return !pop_node(st, stack, hit);
-        }
-    }
     // A tree visits each inner node at most once; the bound only guards
     // against a malformed node array turning into an endless loop.
     if (++st.visits > s.num_nodes + 1) return true;
@@ -299,9 +286,6 @@ RR_D bool trace_step(const DevScene& s, const Ray& r, float tmin, HitRec& hit, T
         if (hk && child < 0) {
             const int first = ~child;
             const int count = k == 0 ? d.z : d.w;
-            if constexpr (Postpone) {
-                if (st.pend_count == 0) { st.pend_first = first; st.pend_count = count; continue; }
-            }
             if (leaf_tris<AnyHit, Count>(s, r, tmin, hit, st, first, count, work)) return true;
         }
     }
@@ -317,11 +301,7 @@ RR_D bool trace_step(const DevScene& s, const Ray& r, float tmin, HitRec& hit, T
     } else if (i1) {
         st.node = d.y;
     } else {
-        if (pop_node(st, stack, hit)) return false;
-        if constexpr (Postpone) {
-            if (st.pend_count > 0) { st.node = -1; return false; }
-        }
-        return true;
+        return !pop_node(st, stack, hit);
     }
     return false;
 }
@@ -424,6 +404,231 @@ RR_D bool trace4(const DevScene& s, const Ray& r, float tmin, float tmax, HitRec
     trav_begin(st, hit, tmax);
     while (!trace_step4<AnyHit, Count>(s, r, tmin, hit, st, stack, work)) {}
     return st.found;
+}
+
+// ── traversal of the quantized trees by whole warps ────────────────────────
+// A child is 16 bytes, one uint4: a word per axis with its lower plane (low
+// half) and its upper plane (high half) on a 15-bit grid over the scene, and
+// its reference (>= 0 an inner node; otherwise a leaf, first triangle << 4 |
+// count under the sign bit). A binary node is 32 bytes, one 256-bit load; a
+// 4-wide node 64 bytes, two.
+//
+// What bounds it: instruction issue (68 % active on the 1M-triangle room's
+// first bounce) and the L1 data path (69 %, node sectors and stack), no
+// longer divergence: 16 of 32 lanes per instruction against 8 with one
+// thread per ray running its leaves' triangle loops inline.
+using u64 = unsigned long long;
+RR_D u64 pack2(float a, float b) { u64 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+RR_D float lo2(u64 v) { return __uint_as_float(uint32_t(v)); }
+RR_D float hi2(u64 v) { return __uint_as_float(uint32_t(v >> 32)); }
+RR_D u64 fma2(u64 a, u64 b, u64 c) {
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+RR_D float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+RR_D float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+RR_D void load32(const void* p, u64& a, u64& b, u64& c, u64& d) {
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
+}
+
+// A ray against the grid. Plane q reads as f = 128 + q / 256 (its 15 bits put
+// into a float's mantissa by one byte permute, whose selector picks the near
+// or the far plane by the direction's sign), and t(q) = f * s + off with s =
+// qscale / d and off = (qbase - o) / d -/+ m. Rounding: s is off by u (2^-24)
+// relative, at most 256 u |s| in t; qbase - o, its product with 1/d and the
+// sum with m by u each, 3 u |qbase - o| / |d|, and the far side's factor once
+// more each; m = 8 u (|qbase - o| + 128 qscale) / |d| is more than all of these, so near planes only move nearer
+// and far ones farther. What is left is relative (the fma, 1/d), and covered
+// by the factor 1.000002 on the far side and 1.00001 on the hit bound, as in
+// box_pair. px..pz keep the shear axes in their upper halves, which the
+// permute does not read.
+struct QuantRay {
+    u64 sx, sy, sz;        // (near, far) slopes
+    u64 ox, oy, oz;        // (near, far) offsets
+    uint32_t px, py, pz;   // byte selectors of the near planes | shear axis << 16
+    uint32_t fx, fy, fz;   // byte selectors of the far planes
+    float3 o;
+    float Sx, Sy, Sz;
+};
+
+RR_D QuantRay make_quant_ray(const DevScene& sc, float3 o, float3 d) {
+    const Ray r = make_ray(o, d);
+    QuantRay q;
+    q.o = o; q.Sx = r.Sx; q.Sy = r.Sy; q.Sz = r.Sz;
+    auto axis = [](float org, float inv, float base, float scale, u64& s, u64& off, uint32_t& p, uint32_t& f) {
+        const float c = base - org;
+        const float a = c * inv;
+        const float m = 4.76837158203125e-7f * fabsf(inv) * (fabsf(c) + 128.0f * scale);
+        const float k = scale * inv;
+        s = pack2(k, k * 1.000002f);
+        off = pack2(a - m, (a + m) * 1.000002f);
+        p = inv >= 0.0f ? 0x7104u : 0x7324u;   // bytes (0, plane, 0x43): 128 + q / 256
+        f = p ^ 0x0220u;
+    };
+    axis(o.x, r.inv.x, sc.qbase.x, sc.qscale.x, q.sx, q.ox, q.px, q.fx);
+    axis(o.y, r.inv.y, sc.qbase.y, sc.qscale.y, q.sy, q.oy, q.py, q.fy);
+    axis(o.z, r.inv.z, sc.qbase.z, sc.qscale.z, q.sz, q.oz, q.pz, q.fz);
+    q.px |= uint32_t(r.kx) << 16;
+    q.py |= uint32_t(r.ky) << 16;
+    q.pz |= uint32_t(r.kz) << 16;
+    return q;
+}
+
+// What a lane does next (LaneTrav::cur): an inner node's index, a leaf (< 0),
+// kPop (take a reference from the stack), kDone (the ray is finished) or
+// kFree (the lane holds no ray).
+constexpr int kPop = 0x7ffffffd, kDone = 0x7ffffffe, kFree = 0x7fffffff;
+
+struct LaneTrav {
+    int cur;
+    int sp;
+    float t, tl;       // hit distance so far and the bound boxes are culled with
+    uint32_t key;      // the hit triangle's flattened id; kNoIndex: none
+    RR_D bool stepping() const { return uint32_t(cur) < uint32_t(kDone); }
+};
+
+template <class Stack>
+RR_D void push_ref(Stack& stack, LaneTrav& st, int ref, float near) {
+    if constexpr (sizeof(typename Stack::Entry) == 4) stack.put(st.sp, ref);
+    else stack.put(st.sp, make_int2(ref, __float_as_int(near)));
+    ++st.sp;
+}
+// The stack's last entry, kPop for one beyond the hit.
+template <class Stack>
+RR_D int pop_ref(const Stack& stack, LaneTrav& st) {
+    --st.sp;
+    if constexpr (sizeof(typename Stack::Entry) == 4) {
+        return stack.get(st.sp);
+    } else {
+        const int2 e = stack.get(st.sp);
+        return __int_as_float(e.y) <= st.tl ? e.x : kPop;
+    }
+}
+// A new ray: the root, above a last entry that ends the traversal.
+template <class Stack>
+RR_D void lane_begin(LaneTrav& st, Stack& stack, float tmax) {
+    st.sp = 0;
+    push_ref(stack, st, kDone, -INFINITY);
+    st.cur = 0;
+    st.t = tmax;
+    st.tl = tmax * 1.00001f;
+    st.key = kNoIndex;
+}
+
+// The two planes of one axis of a child, as (near, far) distances.
+RR_D u64 quant_planes(uint32_t w, uint32_t n, uint32_t f, u64 s, u64 off) {
+    uint32_t a, b;
+    asm("prmt.b32 %0, %1, 0x43000000, %2;" : "=r"(a) : "r"(w), "r"(n));
+    asm("prmt.b32 %0, %1, 0x43000000, %2;" : "=r"(b) : "r"(w), "r"(f));
+    return fma2(pack2(__uint_as_float(a), __uint_as_float(b)), s, off);
+}
+// One child's box; `near` is its entry distance.
+RR_D bool quant_box(const QuantRay& r, u64 wxy, u64 wzr, float tmin, float tl, float& near) {
+    const u64 x = quant_planes(uint32_t(wxy), r.px, r.fx, r.sx, r.ox);
+    const u64 y = quant_planes(uint32_t(wxy >> 32), r.py, r.fy, r.sy, r.oy);
+    const u64 z = quant_planes(uint32_t(wzr), r.pz, r.fz, r.sz, r.oz);
+    near = fmaxf(max3(lo2(x), lo2(y), lo2(z)), tmin);
+    return near <= fminf(min3(hi2(x), hi2(y), hi2(z)), tl);
+}
+
+// One node of the binary tree (a popped reference first): descends into the
+// nearer hit child (any hit: the farther, see trace_step), pushes the other.
+// Leaves are references like inner nodes, so a leaf that turns out to lie
+// beyond a hit is never opened. The visiting order does not change a
+// result: the closest hit is the minimum of (t, key) over all triangles.
+template <bool AnyHit, bool Count, class Stack>
+RR_D void quant_step2(const uint4* nodes, const QuantRay& r, float tmin, LaneTrav& st, Stack& stack, TraceWork* work) {
+    if (st.cur == kPop) {
+        st.cur = pop_ref(stack, st);
+        if (uint32_t(st.cur) >= uint32_t(kPop)) return;
+    }
+    u64 xy0, zr0, xy1, zr1;
+    load32(nodes + size_t(st.cur) * 2, xy0, zr0, xy1, zr1);
+    if (Count) work->nodes++;
+    float n0, n1;
+    const bool h0 = quant_box(r, xy0, zr0, tmin, st.tl, n0), h1 = quant_box(r, xy1, zr1, tmin, st.tl, n1);
+    const int c0 = int(uint32_t(zr0 >> 32)), c1 = int(uint32_t(zr1 >> 32));
+    if (h0 && h1) {
+        const bool one = AnyHit ? n0 <= n1 : n0 > n1;   // child 1 first
+        push_ref(stack, st, one ? c0 : c1, one ? n0 : n1);
+        st.cur = one ? c1 : c0;
+    } else {
+        st.cur = h0 ? c0 : (h1 ? c1 : kPop);
+    }
+}
+
+// One node of the 4-wide tree: the hit children in distance order (any hit
+// farthest first) by a five-comparator network, the first visited next, the
+// others pushed to pop in that order.
+template <bool AnyHit, bool Count, class Stack>
+RR_D void quant_step4(const uint4* nodes, const QuantRay& r, float tmin, LaneTrav& st, Stack& stack, TraceWork* work) {
+    if (st.cur == kPop) {
+        st.cur = pop_ref(stack, st);
+        if (uint32_t(st.cur) >= uint32_t(kPop)) return;
+    }
+    u64 w[8];
+    load32(nodes + size_t(st.cur) * 4, w[0], w[1], w[2], w[3]);
+    load32(nodes + size_t(st.cur) * 4 + 2, w[4], w[5], w[6], w[7]);
+    if (Count) work->nodes++;
+    float key[4];
+    int ref[4];
+    #pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        float near;
+        const bool h = quant_box(r, w[2 * k], w[2 * k + 1], tmin, st.tl, near);
+        key[k] = h ? (AnyHit ? -near : near) : INFINITY;
+        ref[k] = int(uint32_t(w[2 * k + 1] >> 32));
+    }
+    auto cswap = [&](int i, int j) {
+        const bool sw = key[j] < key[i];
+        const float a = key[i];
+        const int c = ref[i];
+        key[i] = sw ? key[j] : a; key[j] = sw ? a : key[j];
+        ref[i] = sw ? ref[j] : c; ref[j] = sw ? c : ref[j];
+    };
+    cswap(0, 1); cswap(2, 3); cswap(0, 2); cswap(1, 3); cswap(1, 2);
+    #pragma unroll
+    for (int k = 3; k >= 1; --k)
+        if (key[k] < INFINITY) push_ref(stack, st, ref[k], key[k]);
+    st.cur = key[0] < INFINITY ? ref[0] : kPop;
+}
+
+// The triangles of the lane's leaf. Closest hit: the lowest (t, key) is kept
+// and handed to hit(u, v, instance, primitive) (float bits), which every
+// later, nearer one follows; any hit: the first one ends the ray.
+template <bool AnyHit, bool Count, class Hit>
+RR_D void quant_leaf(const float4* tris, const QuantRay& q, float tmin, LaneTrav& st, TraceWork* work, Hit hit) {
+    Ray r;
+    r.o = q.o; r.Sx = q.Sx; r.Sy = q.Sy; r.Sz = q.Sz;
+    r.kx = int(q.px >> 16); r.ky = int(q.py >> 16); r.kz = int(q.pz >> 16);
+    int i = int((uint32_t(st.cur) & 0x7fffffffu) >> 4);
+    const int end = i + (st.cur & 15);
+    st.cur = kPop;
+    do {
+        if (Count) work->tris++;
+        const float4 t0 = __ldg(tris + size_t(i) * 3 + 0);
+        const float4 t1 = __ldg(tris + size_t(i) * 3 + 1);
+        const float4 t2 = __ldg(tris + size_t(i) * 3 + 2);
+        float tt, uu, vv;
+        if (intersect_triangle(r, f3(t0.x, t0.y, t0.z), f3(t0.w, t1.x, t1.y), f3(t1.z, t1.w, t2.x), tmin, st.t, tt,
+                               uu, vv)) {
+            const uint32_t key = __float_as_uint(t2.w);
+            if (AnyHit) { st.key = key; st.cur = kDone; return; }
+            if (tt < st.t || key < st.key) {
+                st.t = tt; st.tl = tt * 1.00001f; st.key = key;
+                hit(uu, vv, t2.y, t2.z);
+            }
+        }
+    } while (++i < end);
 }
 
 // Hit attributes (pathtracer.slang:69-118 / restir_di.slang:108-144):

@@ -19,37 +19,39 @@ namespace {
 constexpr int kWaveWords = 8;
 constexpr uint32_t kRis = 0x80000000u;   // ended-candidate flag: it enters resampling
 
+// Tree, SmemS: as traverse_queue's; launched through wave_extend / wave_shadow.
+template <int Tree, int SmemS>
 __global__ void __launch_bounds__(kBlock, 4) wave_extend_kernel(DevScene s, const float4* __restrict__ qa,
                                                                 const float4* __restrict__ qb,
                                                                 float4* __restrict__ hits, uint32_t* c0,
                                                                 float tmin) {
-    traverse_queue<false, false, false>(
+    traverse_queue<false, false, false, Tree, SmemS>(
         s, nullptr, c0[0], c0 + 1, nullptr,
-        [&](uint32_t i, Ray& r, float& tmax) -> uint32_t {
-            r = make_ray(xyz(qa[i]), xyz(qb[i]));
+        [&](uint32_t i, float3& o, float3& d, float& tmax) -> uint32_t {
+            o = xyz(qa[i]);
+            d = xyz(qb[i]);
             tmax = 1e9f;
             return 0u;
         },
-        [&](uint32_t i, bool found, const HitRec& h) {
-            hits[i] = found ? make_float4(h.u, h.v, __uint_as_float(h.inst), __uint_as_float(h.prim))
-                            : make_float4(0.0f, 0.0f, __uint_as_float(kNoIndex), __uint_as_float(kNoIndex));
-        },
-        tmin);
+        StoreHit{hits}, StoreMiss{hits}, tmin);
 }
 
-__global__ void __launch_bounds__(kBlock, 5) wave_shadow_kernel(DevScene s, const float4* __restrict__ sa,
+template <int Tree, int SmemS>
+__global__ void __launch_bounds__(kBlock, 4) wave_shadow_kernel(DevScene s, const float4* __restrict__ sa,
                                                                 const float4* __restrict__ sb,
                                                                 const float4* __restrict__ sc, float4* sum,
                                                                 uint32_t* c0, float tmin) {
-    traverse_queue<true, false, false>(
+    traverse_queue<true, false, false, Tree, SmemS>(
         s, nullptr, c0[2], c0 + 3, nullptr,
-        [&](uint32_t i, Ray& r, float& tmax) -> uint32_t {
+        [&](uint32_t i, float3& o, float3& d, float& tmax) -> uint32_t {
             const float4 b = sb[i];
-            r = make_ray(xyz(sa[i]), xyz(b));
+            o = xyz(sa[i]);
+            d = xyz(b);
             tmax = b.w;
             return 0u;
         },
-        [&](uint32_t i, bool found, const HitRec&) {
+        NoHit{},
+        [&](uint32_t i, bool found) {
             const uint32_t pid = __float_as_uint(sa[i].w);
             const float3 add = found ? f3(0.0f, 0.0f, 0.0f) : xyz(sc[i]);
             const float3 v = xyz(sum[pid]) + add;
@@ -57,6 +59,11 @@ __global__ void __launch_bounds__(kBlock, 5) wave_shadow_kernel(DevScene s, cons
         },
         tmin);
 }
+
+using WaveExtendKernel = decltype(&wave_extend_kernel<4, 12>);
+using WaveShadowKernel = decltype(&wave_shadow_kernel<4, 12>);
+WaveExtendKernel wave_extend(const DevScene& s) { return s.qnodes4 ? wave_extend_kernel<4, 12> : wave_extend_kernel<0, 0>; }
+WaveShadowKernel wave_shadow(const DevScene& s) { return s.qnodes4 ? wave_shadow_kernel<4, 12> : wave_shadow_kernel<0, 0>; }
 
 // The context's wavefront scratch: `arrays` float4 per pixel of state and the
 // counters of `steps` steps (plus one for the rays the last step emits),

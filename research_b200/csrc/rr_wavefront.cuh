@@ -72,102 +72,194 @@ __device__ __forceinline__ void flush_work(const TraceWork& w, unsigned long lon
     if (lane_id() == 0 && (n | t)) { atomicAdd(out, n); atomicAdd(out + 1, t); }
 }
 
-// Queue traversal: each warp takes 32 consecutive queue entries (neighbouring
-// paths after compaction, hence coherent rays) and traces them to the end,
-// then takes the next 32 (the grid is persistent). MinBlocks is the
-// occupancy target handed to the register allocator.
-// `Finish(i, found, hit)` consumes a finished ray; `Load(i, ray, tmax)` makes
-// one and returns its scene index. Multi: a batch of scenes, each ray traced
-// in the scene `table[index]` (the lane binds that scene's node and triangle
-// arrays when it loads the ray); otherwise every ray is traced in `s`. Rays
-// start at t = tmin (the path tracer's 0.001).
-template <int SmemS, int N> struct QueueStackOf { using type = SplitStack<SmemS, kBlock, N>; };
-template <int N> struct QueueStackOf<0, N> { using type = LocalStackN<N>; };
-
+// Queue traversal. `load(i, o, d, tmax)` reads queue entry i and returns its
+// scene index, `hit(i, u, v, instance, primitive)` takes a closest hit (and
+// again every nearer one of the same ray), `done(i, found)` ends the entry.
+// Multi: a batch of scenes, each ray traced in the scene `table[index]` (the
+// lane binds that scene's arrays when it loads the ray); otherwise every ray
+// is traced in `s`. Rays start at t = tmin (the path tracer's 0.001).
+//
+// Tree 4, 2: the quantized 4-wide / binary tree, a warp's lanes in step. Each
+// turn of the loop the warp votes and does one of three things with all
+// lanes that want it:
+//   nodes: kNodeSteps node steps of every lane at an inner node;
+//   leaves: the triangles of every lane waiting at a leaf, once more than
+//     half as many lanes wait there as are at inner nodes (a lane's leaf run
+//     on its own would idle the other 31 for some 100 instructions per
+//     triangle: that took two thirds of the issue slots);
+//   rays: idle lanes finish their rays and take the queue's next entries,
+//     once at most kBusyLanes are busy (neighbouring entries are neighbouring
+//     paths after compaction, so rays stay alike).
+// Measured on the 1080p 4 spp frame of the 1M-triangle room, extension /
+// shadow rays: one thread per ray 16.6 / 11.8 ms; this loop on the
+// full-precision tree, leaf vote 1/4, 1/2, 1: 14.4 / 14.2 / 14.4 and 10.1 /
+// 9.8 / 10.0 ms; with refill at 8, 16, 24 busy lanes 13.8 / 13.7 / 13.4 and
+// 8.8 / 8.1 / 7.8 ms; on the quantized binary tree 12.5 / 6.9 ms; leaves as
+// references and one, two, three node steps a vote 11.5 / 10.8 / 10.5 and
+// 6.4 / 6.1 / 5.8 ms; 4-wide, two steps, stack in shared memory 9.4 / 5.1 ms.
+//
+// Tree 0: the binary tree in full precision, one thread per ray (scenes that
+// the grid does not serve).
+//
 // SmemS > 0: the bottom SmemS stack entries of every thread in shared memory.
-// Wide: the 4-wide tree (trace_step4).
-template <bool AnyHit, bool Count, bool Multi, bool Postpone = false, int SmemS = 0, bool Wide = false, class Load,
-          class Finish>
+template <int SmemS, int N, class E> struct QueueStackOf { using type = SplitStack<SmemS, kBlock, N, E>; };
+template <int N, class E> struct QueueStackOf<0, N, E> { using type = LocalStackN<N, E>; };
+template <bool KeepNear> struct QueueEntryOf { using type = int2; };
+template <> struct QueueEntryOf<false> { using type = int; };
+
+constexpr int kNodeSteps = 2;
+constexpr int kBusyLanes = 24;
+
+template <bool AnyHit, bool Count, bool Multi, int Tree, int SmemS, class Load, class Hit, class Done>
 __device__ __forceinline__ void traverse_queue(const DevScene& s, const DevScene* __restrict__ table, uint32_t count,
-                                               uint32_t* cursor, unsigned long long* work_out, Load load,
-                                               Finish finish, float tmin = 0.001f) {
+                                               uint32_t* cursor, unsigned long long* work_out, Load load, Hit hit,
+                                               Done done, float tmin = 0.001f) {
     TraceWork tw;
-    static_assert(!(Wide && Postpone), "postponed leaves are a binary-tree schedule");
-    typename QueueStackOf<SmemS, Wide ? kStackSize4 : kStackSize>::type stack;   // (node, near distance) entries
+    // an any-hit ray's bound never moves: its entries need no distance
+    using Entry = typename QueueEntryOf<Tree == 0 || !AnyHit>::type;
+    typename QueueStackOf<SmemS, Tree == 4 ? kStackSize4 : kStackSize, Entry>::type stack;
     if constexpr (SmemS > 0) {
-        __shared__ int2 stack_smem[SmemS * kBlock];
+        __shared__ Entry stack_smem[SmemS * kBlock];
         stack.col = stack_smem + threadIdx.x;
     }
-    DevScene ls{};           // Multi: the current ray's scene (traversal fields)
-    auto bind = [&](uint32_t sid) {
-        if constexpr (Multi) {
-            ls.nodes = table[sid].nodes;
-            ls.tris = table[sid].tris;
-            ls.num_nodes = table[sid].num_nodes;
-            ls.nodes4 = table[sid].nodes4;
-            ls.num_nodes4 = table[sid].num_nodes4;
+    if constexpr (Tree == 0) {
+        DevScene ls{};
+        while (true) {
+            uint32_t base = 0;
+            if (lane_id() == 0) base = atomicAdd(cursor, 32u);
+            base = __shfl_sync(kFull, base, 0);
+            if (base >= count) break;
+            const uint32_t i = base + lane_id();
+            if (i < count) {
+                float3 o, d;
+                float tmax;
+                const uint32_t sid = load(i, o, d, tmax);
+                if constexpr (Multi) {
+                    ls.nodes = table[sid].nodes;
+                    ls.tris = table[sid].tris;
+                    ls.num_nodes = table[sid].num_nodes;
+                }
+                const Ray r = make_ray(o, d);
+                HitRec h; TravState st;
+                trav_begin(st, h, tmax);
+                while (!trace_step<AnyHit, Count>(Multi ? ls : s, r, tmin, h, st, stack, &tw)) {}
+                if (!AnyHit && st.found) hit(i, h.u, h.v, __uint_as_float(h.inst), __uint_as_float(h.prim));
+                done(i, st.found);
+            }
         }
-    };
-    auto step = [&](const Ray& r, HitRec& h, TravState& st) -> bool {
-        const DevScene& sc = Multi ? ls : s;
-        if constexpr (Wide) return trace_step4<AnyHit, Count>(sc, r, tmin, h, st, stack, &tw);
-        else return trace_step<AnyHit, Count, Postpone>(sc, r, tmin, h, st, stack, &tw);
-    };
-    while (true) {
-        uint32_t base = 0;
-        if (lane_id() == 0) base = atomicAdd(cursor, 32u);
-        base = __shfl_sync(kFull, base, 0);
-        if (base >= count) break;
-        const uint32_t i = base + lane_id();
-        if (i < count) {
-            Ray r; float tmax;
-            bind(load(i, r, tmax));
-            HitRec h; TravState st;
-            trav_begin(st, h, tmax);
-            while (!step(r, h, st)) {}
-            finish(i, st.found, h);
+    } else {
+        const uint4* nodes = Tree == 4 ? s.qnodes4 : s.qnodes;
+        const float4* tris = s.tris;
+        QuantRay r;
+        LaneTrav st;
+        st.cur = kFree;
+        uint32_t i = 0;
+        bool more = true;   // the queue may hold entries not taken yet
+        while (true) {
+            const uint32_t leafm = __ballot_sync(kFull, st.cur < 0);
+            const uint32_t nodem = __ballot_sync(kFull, st.stepping());
+            if ((leafm | nodem) == 0 || (more && __popc(leafm | nodem) <= kBusyLanes)) {
+                const bool idle = st.cur >= kDone;
+                if (st.cur == kDone) {
+                    done(i, st.key != kNoIndex);
+                    st.cur = kFree;
+                }
+                if (!more) break;   // nobody is busy
+                const uint32_t idlem = __ballot_sync(kFull, idle);
+                uint32_t base = 0;
+                if (lane_id() == 0) base = atomicAdd(cursor, __popc(idlem));
+                base = __shfl_sync(kFull, base, 0);
+                more = base + __popc(idlem) < count;
+                if (idle) {
+                    i = base + __popc(idlem & ((1u << lane_id()) - 1u));
+                    if (i < count) {
+                        float3 o, d;
+                        float tmax;
+                        const uint32_t sid = load(i, o, d, tmax);
+                        if constexpr (Multi) {
+                            nodes = Tree == 4 ? table[sid].qnodes4 : table[sid].qnodes;
+                            tris = table[sid].tris;
+                            r = make_quant_ray(table[sid], o, d);
+                        } else {
+                            r = make_quant_ray(s, o, d);
+                        }
+                        lane_begin(st, stack, tmax);
+                    }
+                }
+                continue;
+            }
+            if (nodem == 0 || __popc(leafm) * 2 > __popc(nodem)) {
+                if (st.cur < 0)
+                    quant_leaf<AnyHit, Count>(tris, r, tmin, st, &tw, [&](float u, float v, float inst, float prim) {
+                        hit(i, u, v, inst, prim);
+                    });
+            } else {
+                #pragma unroll
+                for (int k = 0; k < kNodeSteps; ++k)
+                    if (st.stepping()) {
+                        if constexpr (Tree == 4) quant_step4<AnyHit, Count>(nodes, r, tmin, st, stack, &tw);
+                        else quant_step2<AnyHit, Count>(nodes, r, tmin, st, stack, &tw);
+                    }
+            }
         }
     }
     if (Count) flush_work(tw, work_out);
 }
 
-template <bool Count, int MinBlocks, bool Postpone = false, int SmemS = 0, bool Wide = false>
+// Closest hits of the ray queue (a, b) into `hits`: (u, v, instance,
+// primitive), all ones for a miss.
+struct StoreHit {
+    float4* hits;
+    __device__ __forceinline__ void operator()(uint32_t i, float u, float v, float inst, float prim) const {
+        hits[i] = make_float4(u, v, inst, prim);
+    }
+};
+struct StoreMiss {
+    float4* hits;
+    __device__ __forceinline__ void operator()(uint32_t i, bool found) const {
+        if (!found) hits[i] = make_float4(0.0f, 0.0f, __uint_as_float(kNoIndex), __uint_as_float(kNoIndex));
+    }
+};
+struct NoHit {
+    __device__ __forceinline__ void operator()(uint32_t, float, float, float, float) const {}
+};
+
+template <bool Count, int MinBlocks, int Tree, int SmemS>
 __global__ void __launch_bounds__(kBlock, MinBlocks) extend_kernel(DevScene s, const float4* __restrict__ qa,
                                                                    const float4* __restrict__ qb,
                                                                    float4* __restrict__ hits,
                                                                    const uint32_t* count_ptr, uint32_t* cursor,
                                                                    unsigned long long* work_out) {
-    traverse_queue<false, Count, false, Postpone, SmemS, Wide>(
+    traverse_queue<false, Count, false, Tree, SmemS>(
         s, nullptr, *count_ptr, cursor, work_out,
-        [&](uint32_t i, Ray& r, float& tmax) -> uint32_t {
-            const float4 a = qa[i], b = qb[i];
-            r = make_ray(f3(a.x, a.y, a.z), f3(b.x, b.y, b.z));
+        [&](uint32_t i, float3& o, float3& d, float& tmax) -> uint32_t {
+            o = xyz(qa[i]);
+            d = xyz(qb[i]);
             tmax = 1e9f;
             return 0u;
         },
-        [&](uint32_t i, bool found, const HitRec& h) {
-            hits[i] = found ? make_float4(h.u, h.v, __uint_as_float(h.inst), __uint_as_float(h.prim))
-                            : make_float4(0.0f, 0.0f, __uint_as_float(kNoIndex), __uint_as_float(kNoIndex));
-        });
+        StoreHit{hits}, StoreMiss{hits});
 }
 
 // Any-hit shadow rays; unoccluded NEE contributions are added to the image.
-template <bool Count, int MinBlocks, bool Postpone = false, int SmemS = 0, bool Wide = false>
+template <bool Count, int MinBlocks, int Tree, int SmemS>
 __global__ void __launch_bounds__(kBlock, MinBlocks) shadow_kernel(DevScene s, const float4* __restrict__ sa,
                                                                    const float4* __restrict__ sb,
                                                                    const float4* __restrict__ sc,
                                                                    float4* __restrict__ out,
                                                                    const uint32_t* count_ptr, uint32_t* cursor,
                                                                    unsigned long long* work_out) {
-    traverse_queue<true, Count, false, Postpone, SmemS, Wide>(
+    traverse_queue<true, Count, false, Tree, SmemS>(
         s, nullptr, *count_ptr, cursor, work_out,
-        [&](uint32_t i, Ray& r, float& tmax) -> uint32_t {
-            const float4 a = sa[i], b = sb[i];
-            r = make_ray(f3(a.x, a.y, a.z), f3(b.x, b.y, b.z));
+        [&](uint32_t i, float3& o, float3& d, float& tmax) -> uint32_t {
+            const float4 b = sb[i];
+            o = xyz(sa[i]);
+            d = xyz(b);
             tmax = b.w;
             return 0u;
         },
-        [&](uint32_t i, bool found, const HitRec&) {
+        NoHit{},
+        [&](uint32_t i, bool found) {
             if (!found) {
                 const float4 c = sc[i];
                 const uint32_t pid = __float_as_uint(sa[i].w);
@@ -228,7 +320,7 @@ __global__ void __launch_bounds__(kBlock) raygen_batch_kernel(const BatchEntry* 
     qc[slot] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(sid));
 }
 
-template <bool Count, int MinBlocks, bool Postpone = false, int SmemS = 0, bool Wide = false>
+template <bool Count, int MinBlocks, int Tree, int SmemS>
 __global__ void __launch_bounds__(kBlock, MinBlocks) extend_batch_kernel(const DevScene* __restrict__ table,
                                                                          const float4* __restrict__ qa,
                                                                          const float4* __restrict__ qb,
@@ -237,21 +329,18 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) extend_batch_kernel(const D
                                                                          const uint32_t* count_ptr, uint32_t* cursor,
                                                                          unsigned long long* work_out) {
     const DevScene none{};
-    traverse_queue<false, Count, true, Postpone, SmemS, Wide>(
+    traverse_queue<false, Count, true, Tree, SmemS>(
         none, table, *count_ptr, cursor, work_out,
-        [&](uint32_t i, Ray& r, float& tmax) -> uint32_t {
-            const float4 a = qa[i], b = qb[i];
-            r = make_ray(f3(a.x, a.y, a.z), f3(b.x, b.y, b.z));
+        [&](uint32_t i, float3& o, float3& d, float& tmax) -> uint32_t {
+            o = xyz(qa[i]);
+            d = xyz(qb[i]);
             tmax = 1e9f;
             return __float_as_uint(qc[i].w);
         },
-        [&](uint32_t i, bool found, const HitRec& h) {
-            hits[i] = found ? make_float4(h.u, h.v, __uint_as_float(h.inst), __uint_as_float(h.prim))
-                            : make_float4(0.0f, 0.0f, __uint_as_float(kNoIndex), __uint_as_float(kNoIndex));
-        });
+        StoreHit{hits}, StoreMiss{hits});
 }
 
-template <bool Count, int MinBlocks, bool Postpone = false, int SmemS = 0, bool Wide = false>
+template <bool Count, int MinBlocks, int Tree, int SmemS>
 __global__ void __launch_bounds__(kBlock, MinBlocks) shadow_batch_kernel(const DevScene* __restrict__ table,
                                                                          float4* const* __restrict__ outs,
                                                                          const float4* __restrict__ sa,
@@ -260,15 +349,17 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) shadow_batch_kernel(const D
                                                                          const uint32_t* count_ptr, uint32_t* cursor,
                                                                          unsigned long long* work_out) {
     const DevScene none{};
-    traverse_queue<true, Count, true, Postpone, SmemS, Wide>(
+    traverse_queue<true, Count, true, Tree, SmemS>(
         none, table, *count_ptr, cursor, work_out,
-        [&](uint32_t i, Ray& r, float& tmax) -> uint32_t {
-            const float4 a = sa[i], b = sb[i];
-            r = make_ray(f3(a.x, a.y, a.z), f3(b.x, b.y, b.z));
+        [&](uint32_t i, float3& o, float3& d, float& tmax) -> uint32_t {
+            const float4 b = sb[i];
+            o = xyz(sa[i]);
+            d = xyz(b);
             tmax = b.w;
             return __float_as_uint(sc[i].w);
         },
-        [&](uint32_t i, bool found, const HitRec&) {
+        NoHit{},
+        [&](uint32_t i, bool found) {
             if (!found) {
                 const float4 c = sc[i];
                 const uint32_t pid = __float_as_uint(sa[i].w);
@@ -284,67 +375,41 @@ using BatchQueueKernel = void (*)(const DevScene*, const float4*, const float4*,
                                   const uint32_t*, uint32_t*, unsigned long long*);
 using BatchShadowKernel = void (*)(const DevScene*, float4* const*, const float4*, const float4*, const float4*,
                                    const uint32_t*, uint32_t*, unsigned long long*);
-// Variant 0 of the batch extend kernel asks for 4 blocks per SM: left free,
-// the per-ray scene binding takes it to 68 registers (3 blocks of 256 per
-// SM), where the single-scene kernel settles at 64 (4 blocks).
-template <bool Count>
-BatchQueueKernel extend_batch_variant(int v) {
-    switch (v) {
-    case 1: return extend_batch_kernel<Count, 5>;
-    case 2: return extend_batch_kernel<Count, 1, false, 8>;
-    case 3: return extend_batch_kernel<Count, 1, false, 0, true>;
-    case 4: return extend_batch_kernel<Count, 1, false, 8, true>;
-    case 5: return extend_batch_kernel<Count, 5, false, 8>;
-    case 6: return extend_batch_kernel<Count, 3, false, 8, true>;
-    case 7: return extend_batch_kernel<Count, 4, true>;
-    default: return extend_batch_kernel<Count, 4>;
+// Traversal kernel variants (rr_pathtracer_set_variants): MinBlocks x tree x
+// stack entries in shared memory. A scene whose trees are not quantized is
+// traced by kVariantFull's kernel whatever the variant. kVariantDefault is
+// the fastest on the 1M-triangle room (extension / shadow rays of the 1080p
+// frame 9.4 / 5.1 ms; 9.5 / 5.3 ms with the whole stack in local memory;
+// binary tree 10.4 / 5.5 ms).
+constexpr int kVariantFull = 7, kVariantDefault = 4;
+#define RR_TRAVERSAL_VARIANTS(kernel, v)                   \
+    switch (v) {                                           \
+    case 0: return kernel<Count, 4, 2, 8>;                 \
+    case 1: return kernel<Count, 5, 2, 0>;                 \
+    case 2: return kernel<Count, 4, 2, 0>;                 \
+    case 3: return kernel<Count, 4, 4, 0>;                 \
+    case 5: return kernel<Count, 5, 2, 12>;                \
+    case 6: return kernel<Count, 5, 4, 8>;                 \
+    case kVariantFull: return kernel<Count, 4, 0, 0>;      \
+    default: return kernel<Count, 4, 4, 12>;               \
     }
-}
-template <bool Count>
-BatchShadowKernel shadow_batch_variant(int v) {
-    switch (v) {
-    case 1: return shadow_batch_kernel<Count, 5>;
-    case 2: return shadow_batch_kernel<Count, 1, false, 8>;
-    case 3: return shadow_batch_kernel<Count, 1, false, 0, true>;
-    case 4: return shadow_batch_kernel<Count, 1, false, 8, true>;
-    case 5: return shadow_batch_kernel<Count, 5, false, 8>;
-    case 6: return shadow_batch_kernel<Count, 3, false, 8, true>;
-    case 7: return shadow_batch_kernel<Count, 4, true>;
-    default: return shadow_batch_kernel<Count, 1>;
-    }
-}
 
-// Traversal kernel variants: schedule x occupancy target x stack placement.
+template <bool Count>
+BatchQueueKernel extend_batch_variant(int v) { RR_TRAVERSAL_VARIANTS(extend_batch_kernel, v) }
+template <bool Count>
+BatchShadowKernel shadow_batch_variant(int v) { RR_TRAVERSAL_VARIANTS(shadow_batch_kernel, v) }
+
 using QueueKernel = void (*)(DevScene, const float4*, const float4*, float4*, const uint32_t*, uint32_t*,
                              unsigned long long*);
 using ShadowKernel = void (*)(DevScene, const float4*, const float4*, const float4*, float4*, const uint32_t*,
                               uint32_t*, unsigned long long*);
 template <bool Count>
-QueueKernel extend_variant(int v) {
-    switch (v) {
-    case 1: return extend_kernel<Count, 5>;
-    case 2: return extend_kernel<Count, 1, false, 8>;
-    case 3: return extend_kernel<Count, 1, false, 0, true>;
-    case 4: return extend_kernel<Count, 1, false, 8, true>;
-    case 5: return extend_kernel<Count, 5, false, 8>;
-    case 6: return extend_kernel<Count, 3, false, 8, true>;
-    case 7: return extend_kernel<Count, 4, true>;
-    default: return extend_kernel<Count, 1>;
-    }
-}
+QueueKernel extend_variant(int v) { RR_TRAVERSAL_VARIANTS(extend_kernel, v) }
 template <bool Count>
-ShadowKernel shadow_variant(int v) {
-    switch (v) {
-    case 1: return shadow_kernel<Count, 5>;
-    case 2: return shadow_kernel<Count, 1, false, 8>;
-    case 3: return shadow_kernel<Count, 1, false, 0, true>;
-    case 4: return shadow_kernel<Count, 1, false, 8, true>;
-    case 5: return shadow_kernel<Count, 5, false, 8>;
-    case 6: return shadow_kernel<Count, 3, false, 8, true>;
-    case 7: return shadow_kernel<Count, 4, true>;
-    default: return shadow_kernel<Count, 1>;
-    }
-}
+ShadowKernel shadow_variant(int v) { RR_TRAVERSAL_VARIANTS(shadow_kernel, v) }
+
+// The variant a scene's rays run: the asked one, or the full-precision form.
+int variant_for(const DevScene& s, int v) { return s.qnodes4 ? v : kVariantFull; }
 
 int persistent_grid(const rr_ctx* ctx, const void* kernel) {
     int per_sm = 0;

@@ -283,6 +283,12 @@ rr_status rr_scene_create(rr_ctx* ctx, const rr_scene_desc* d, rr_scene** out) {
     s->dev.field = reinterpret_cast<type>(p);
     RR_UP(bvh.nodes.data(), bvh.nodes.size() * sizeof(float4), nodes, const float4*);
     RR_UP(bvh.nodes4.data(), bvh.nodes4.size() * sizeof(float4), nodes4, const float4*);
+    if (!bvh.qnodes.empty()) {
+        RR_UP(bvh.qnodes.data(), bvh.qnodes.size() * sizeof(uint4), qnodes, const uint4*);
+        RR_UP(bvh.qnodes4.data(), bvh.qnodes4.size() * sizeof(uint4), qnodes4, const uint4*);
+        s->dev.qbase = make_float3(bvh.qbase[0], bvh.qbase[1], bvh.qbase[2]);
+        s->dev.qscale = make_float3(bvh.qscale[0], bvh.qscale[1], bvh.qscale[2]);
+    }
     RR_UP(trirec.data(), trirec.size() * sizeof(float4), tris, const float4*);
     RR_UP(d->vertices, size_t(d->vertex_count) * sizeof(GpuVertex), vertices, const float4*);
     RR_UP(d->indices, size_t(d->index_count) * 4, indices, const uint32_t*);

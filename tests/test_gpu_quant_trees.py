@@ -1,0 +1,83 @@
+"""GPU tests of the queue traversal over the quantized trees, at the scenes
+where its grid and its dispatch can go wrong. The tolerance is zero: a box
+only decides which triangles are tested, so the images are the oracle's bits
+whichever tree is walked (variant 7 walks the full-precision one)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _scaled(arrays, scale, shift):
+    """The arrays with every instance scaled per axis, then moved."""
+    a = {k: v.copy() for k, v in arrays.items()}
+    for inst in a["instances"]:
+        m = inst["transform"].reshape(4, 4)
+        m[:3] = np.asarray(scale, np.float32)[:, None] * m[:3]
+        m[:3, 3] += np.asarray(shift, np.float32)
+    a["lights"]["position"] = a["lights"]["position"] * np.asarray(scale, np.float32) + np.asarray(shift, np.float32)
+    return a
+
+
+def _one_mesh(arrays, keep):
+    """Only the first `keep` triangles of the first instance's mesh: one leaf for a few."""
+    a = {k: v.copy() for k, v in arrays.items()}
+    a["instances"] = a["instances"][:1]
+    m = int(a["instances"]["mesh_index"][0])
+    a["meshes"]["index_count"][m] = 3 * keep
+    return a
+
+
+def _outlier(arrays, distance):
+    """One instance more, far away: the grid's step grows with the distance."""
+    a = {k: v.copy() for k, v in arrays.items()}
+    far = a["instances"][:1].copy()
+    far[0]["transform"].reshape(4, 4)[:3, 3] += np.float32(distance)
+    a["instances"] = np.concatenate([a["instances"], far])
+    return a
+
+
+CASES = {
+    "cornell": lambda c: (c, (1, 1, 1), (0, 0, 0)),
+    "root_is_a_leaf": lambda c: (_one_mesh(c, 1), (1, 1, 1), (0, 0, 0)),
+    "two_coplanar_triangles": lambda c: (_one_mesh(c, 2), (1, 1, 1), (0, 0, 0)),
+    "large_coordinates": lambda c: (_scaled(c, (1, 1, 1), (3e4, -2e4, 5e4)), (1, 1, 1), (3e4, -2e4, 5e4)),
+    "tiny": lambda c: (_scaled(c, (1e-3, 1e-3, 1e-3), (0, 0, 0)), (1e-3, 1e-3, 1e-3), (0, 0, 0)),
+    "anisotropic": lambda c: (_scaled(c, (50, 0.02, 1), (0, 0, 0)), (50, 0.02, 1), (0, 0, 0)),
+    "outlier_near": lambda c: (_outlier(c, 30.0), (1, 1, 1), (0, 0, 0)),
+    "outlier_far": lambda c: (_outlier(c, 1e7), (1, 1, 1), (0, 0, 0)),
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_quantized_traversal_bit_exact(rr, O, ctx, torch_cuda, name):
+    torch = torch_cuda
+    base = rr.HostScene.cornell(0).arrays
+    arrays, scale, shift = CASES[name](base)
+    scene = rr.Scene(ctx, arrays)
+    oscene = O.OracleScene(arrays, use_bvh=False)
+    s, t = np.asarray(scale, np.float64), np.asarray(shift, np.float64)
+    # an odd image, and an axis-parallel view: zero direction components
+    cam = rr.camera_data(rr.camera_desc(45, 31, eye=tuple(np.array([0.0, 1.0, 3.2]) * s + t),
+                                        center=tuple(np.array([0.0, 1.0, 0.0]) * s + t)))
+    ref, _ = O.pathtrace(oscene, cam, 5, 4, 2)
+    st = torch.cuda.current_stream().cuda_stream
+    L = rr.lib()
+    try:
+        for v in range(rr.PT_VARIANT_COUNT):
+            ctx.check(L.rr_pathtracer_set_variants(ctx.handle, v, v))
+            for flags in (0, rr.PT_FLAG_COUNT_TRAVERSAL):
+                out = torch.empty((2, 31, 45, 4), device="cuda")
+                p = rr.PtParams(5, 4, 2, flags)
+                ctx.check(L.rr_pathtracer_execute(ctx.handle, scene.handle, C.byref(cam), C.byref(p), out.data_ptr(),
+                                                  st))
+                got = out.cpu().numpy()
+                np.testing.assert_array_equal(got.view(np.uint32), ref.view(np.uint32), err_msg=f"variant {v}")
+            stats = rr.PtStats()
+            ctx.check(L.rr_pathtracer_stats(ctx.handle, C.byref(stats), 1))
+            assert stats.extension_nodes >= stats.extension_rays   # every ray visits the root
+    finally:
+        ctx.check(L.rr_pathtracer_set_variants(ctx.handle, 0, 0))
+        scene.close()
