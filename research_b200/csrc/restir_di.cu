@@ -99,21 +99,16 @@ RR_D float di_p_hat(const DevScene& s, uint32_t sel, float3 pos, float3 n) {
     else return compute_p_hat(s, sel, pos, n);
 }
 
-RR_D bool pixel_of(const GpuCameraData& cam, uint32_t& x, uint32_t& y) {
-    x = blockIdx.x * 16 + (threadIdx.x & 15);
-    y = blockIdx.y * 8 + (threadIdx.x >> 4);
-    return x < cam.screen_width && y < cam.screen_height;
-}
-
-// cs_initial (restir_di.slang:186-262). The initial and spatial kernels run
-// 10 blocks of 128 threads per SM (48 registers, a few spilled): 251.9
-// against 250.8 Mpaths/s for the bench frame with 8 blocks (64 registers),
-// 250.6 with 6.
-template <bool Emit>
-__global__ void __launch_bounds__(128, 10) di_initial_kernel(DevScene s, DiLaunch L, float4* __restrict__ gpos,
+// cs_initial (restir_di.slang:186-262). The initial and spatial kernels trace
+// with trace_lanes (Tree as there) and run 8 blocks of 128 threads per SM (64
+// registers): 1.96 ms for a 1080p frame of the 1M-triangle room (2.61 ms with
+// one thread per ray on the full-precision tree); 2.06 ms with 10 blocks,
+// 2.09 ms with 6.
+template <bool Emit, int Tree>
+__global__ void __launch_bounds__(128, 8) di_initial_kernel(DevScene s, DiLaunch L, float4* __restrict__ gpos,
                                                          float4* __restrict__ gnrm, float4* __restrict__ res) {
     uint32_t x, y;
-    if (!pixel_of(L.cam, x, y)) return;
+    if (!tile_pixel(L.cam, x, y)) return;
     const size_t i = size_t(y) * L.cam.screen_width + x;
     uint32_t seed = make_seed(x, y, L.frame_seed);
     const float jx = rand_float(seed);
@@ -121,7 +116,7 @@ __global__ void __launch_bounds__(128, 10) di_initial_kernel(DevScene s, DiLaunc
     const float3 d = primary_dir(L.cam, float(x) + jx, float(y) + jy);
     const float3 o = f3(L.cam.position[0], L.cam.position[1], L.cam.position[2]);
     HitRec h;
-    if (!trace<false>(s, make_ray(o, d), 0.001f, 1e9f, h)) {
+    if (!trace_lanes<false, Tree>(s, o, d, 0.001f, 1e9f, h)) {
         gpos[i] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
         gnrm[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         res[i] = make_float4(__uint_as_float(kNoIndex), 0.0f, 0.0f, __uint_as_float(0u));
@@ -171,7 +166,7 @@ __global__ void __launch_bounds__(128) di_temporal_kernel(DevScene s, DiLaunch L
                                                           const float4* __restrict__ gnrm, float4* __restrict__ res,
                                                           const float4* __restrict__ prev) {
     uint32_t x, y;
-    if (!pixel_of(L.cam, x, y)) return;
+    if (!tile_pixel(L.cam, x, y)) return;
     const size_t i = size_t(y) * L.cam.screen_width + x;
     const float4 gp = gpos[i];
     if (gp.w < 0.0f) return;
@@ -208,13 +203,13 @@ __global__ void __launch_bounds__(128) di_temporal_kernel(DevScene s, DiLaunch L
 }
 
 // cs_spatial_shade (restir_di.slang:339-472)
-template <bool Emit>
-__global__ void __launch_bounds__(128, 10) di_spatial_shade_kernel(DevScene s, DiLaunch L, const float4* __restrict__ gpos,
+template <bool Emit, int Tree>
+__global__ void __launch_bounds__(128, 8) di_spatial_shade_kernel(DevScene s, DiLaunch L, const float4* __restrict__ gpos,
                                                                const float4* __restrict__ gnrm,
                                                                const float4* __restrict__ res,
                                                                float4* __restrict__ out) {
     uint32_t x, y;
-    if (!pixel_of(L.cam, x, y)) return;
+    if (!tile_pixel(L.cam, x, y)) return;
     const uint32_t W = L.cam.screen_width, H = L.cam.screen_height;
     const size_t i = size_t(y) * W + x;
     const float4 gp = gpos[i];
@@ -228,7 +223,7 @@ __global__ void __launch_bounds__(128, 10) di_spatial_shade_kernel(DevScene s, D
     const float4 gn = gnrm[i];
     const float3 n = xyz(gn);
     const uint32_t mat = __float_as_uint(gn.w);
-    const float4 m0 = __ldg(s.materials + mat * 2), m1 = __ldg(s.materials + mat * 2 + 1);
+    const float4 m1 = __ldg(s.materials + mat * 2 + 1);
     if (m1.x > 0.0f || m1.y > 0.0f || m1.z > 0.0f) {
         out[i] = make_float4(m1.x, m1.y, m1.z, 1.0f);
         return;
@@ -264,30 +259,26 @@ __global__ void __launch_bounds__(128, 10) di_spatial_shade_kernel(DevScene s, D
             r_W = (ph_y > 1e-10f) ? (r_wsum / (float(r_M) * ph_y)) : 0.0f;
         }
     }
-    float3 o = f3(0.0f, 0.0f, 0.0f);
+    // the selected sample's direction, distance and irradiance; one shadow ray
+    float3 l = f3(0.0f, 0.0f, 0.0f), irr = l;
+    float dist = 0.0f;
+    bool shade;
     uint32_t li = r_sel;
     bool gpu_light;
     if constexpr (Emit) {
         gpu_light = false;
+        shade = false;
         if (r_sel != kNoIndex && NA > 0 && r_W > 0.0f) {
             const DiLightSample ds = di_decode(s, r_sel);
             if (ds.emitter) {
                 // a point on an emissive triangle: irradiance Le |cos_y| / d^2
                 const float3 to = ds.y - pos;
-                const float dist = length(to);
-                const float3 l = to / mx(dist, 1e-6f);
+                dist = length(to);
+                l = to / mx(dist, 1e-6f);
                 const float dd = mx(dist * dist, 1e-6f);
                 const float cos_y = fabsf(dot(ds.ny, l));
-                const float3 irr = ds.Le * (cos_y / dd);
-                const float ndl = mx(dot(n, l), 0.0f);
-                if (ndl > 0.0f) {
-                    HitRec h;
-                    if (!trace<true>(s, make_ray(pos + n * 1e-4f, l), 0.001f, dist - 0.01f, h)) {
-                        const float3 wo = normalize(f3(L.cam.position[0], L.cam.position[1], L.cam.position[2]) - pos);
-                        const float3 bv = brdf_eval(n, wo, l, f3(m0.x, m0.y, m0.z), m0.w, m1.w);
-                        o = ((bv * irr) * ndl) * r_W;
-                    }
-                }
+                irr = ds.Le * (cos_y / dd);
+                shade = true;
             } else {
                 li = ds.li;
                 gpu_light = N > 0;
@@ -297,12 +288,12 @@ __global__ void __launch_bounds__(128, 10) di_spatial_shade_kernel(DevScene s, D
         // r_sel < N guards the light fetch for reservoirs that were never
         // written by this scene; valid reservoirs always satisfy it.
         gpu_light = r_sel != kNoIndex && r_sel < N && r_W > 0.0f && N > 0;
+        shade = false;
     }
     if (gpu_light) {
         const float4 l0 = __ldg(s.lights + li * 3);
         const float4 l1 = __ldg(s.lights + li * 3 + 1);
         const float4 l2 = __ldg(s.lights + li * 3 + 2);
-        float3 l, irr; float dist;
         if (__float_as_uint(l0.w) == 0u) {
             const float3 to = f3(l0.x, l0.y, l0.z) - pos;
             dist = length(to);
@@ -314,14 +305,17 @@ __global__ void __launch_bounds__(128, 10) di_spatial_shade_kernel(DevScene s, D
             dist = 1e9f;
             irr = f3(l2.x, l2.y, l2.z) * l2.w;
         }
-        const float ndl = mx(dot(n, l), 0.0f);
-        if (ndl > 0.0f) {
-            HitRec h;
-            if (!trace<true>(s, make_ray(pos + n * 1e-4f, l), 0.001f, dist - 0.01f, h)) {
-                const float3 wo = normalize(f3(L.cam.position[0], L.cam.position[1], L.cam.position[2]) - pos);
-                const float3 bv = brdf_eval(n, wo, l, f3(m0.x, m0.y, m0.z), m0.w, m1.w);
-                o = ((bv * irr) * ndl) * r_W;
-            }
+        shade = true;
+    }
+    float3 o = f3(0.0f, 0.0f, 0.0f);
+    const float ndl = mx(dot(n, l), 0.0f);
+    if (shade && ndl > 0.0f) {
+        HitRec h;
+        if (!trace_lanes<true, Tree>(s, pos + n * 1e-4f, l, 0.001f, dist - 0.01f, h)) {
+            const float3 wo = normalize(f3(L.cam.position[0], L.cam.position[1], L.cam.position[2]) - pos);
+            const float4 m0 = __ldg(s.materials + mat * 2);
+            const float3 bv = brdf_eval(n, wo, l, f3(m0.x, m0.y, m0.z), m0.w, m1.w);
+            o = ((bv * irr) * ndl) * r_W;
         }
     }
     out[i] = make_float4(o.x, o.y, o.z, 1.0f);
@@ -365,8 +359,10 @@ extern "C" rr_status rr_restir_di_initial(rr_ctx* ctx, const rr_scene* scene, co
     if (st != RR_OK) return st;
     if (!gpos || !gnrm || !res) return rr_fail(ctx, RR_ERR_INVALID_ARGUMENT, "null buffer");
     RR_TRY_CUDA(ctx, cudaSetDevice(ctx->device));
-    const auto di_initial_kernel_f = (p->flags & RR_DI_FLAG_EMITTERS) ? di_initial_kernel<true> : di_initial_kernel<false>;
-    di_initial_kernel_f<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    const bool quant = scene->dev.qnodes4 != nullptr;
+    const auto kernel = (p->flags & RR_DI_FLAG_EMITTERS) ? (quant ? di_initial_kernel<true, 4> : di_initial_kernel<true, 0>)
+                                                         : (quant ? di_initial_kernel<false, 4> : di_initial_kernel<false, 0>);
+    kernel<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(
         scene->dev, make_launch(cam, p), reinterpret_cast<float4*>(gpos), reinterpret_cast<float4*>(gnrm),
         reinterpret_cast<float4*>(res));
     RR_CHECK_LAUNCH(ctx);
@@ -401,8 +397,10 @@ extern "C" rr_status rr_restir_di_spatial_shade(rr_ctx* ctx, const rr_scene* sce
     if (st != RR_OK) return st;
     if (!gpos || !gnrm || !res || !out) return rr_fail(ctx, RR_ERR_INVALID_ARGUMENT, "null buffer");
     RR_TRY_CUDA(ctx, cudaSetDevice(ctx->device));
-    const auto di_spatial_shade_kernel_f = (p->flags & RR_DI_FLAG_EMITTERS) ? di_spatial_shade_kernel<true> : di_spatial_shade_kernel<false>;
-    di_spatial_shade_kernel_f<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    const bool quant = scene->dev.qnodes4 != nullptr;
+    const auto kernel = (p->flags & RR_DI_FLAG_EMITTERS) ? (quant ? di_spatial_shade_kernel<true, 4> : di_spatial_shade_kernel<true, 0>)
+                                                         : (quant ? di_spatial_shade_kernel<false, 4> : di_spatial_shade_kernel<false, 0>);
+    kernel<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(
         scene->dev, make_launch(cam, p), reinterpret_cast<const float4*>(gpos),
         reinterpret_cast<const float4*>(gnrm), reinterpret_cast<const float4*>(res),
         reinterpret_cast<float4*>(out));

@@ -91,9 +91,10 @@ RR_D float gi_source_pdf(float3 pp, float3 pn, float3 spos) {
 }
 
 // cs_initial (restir_gi.slang:568-686)
+template <int Tree>
 __global__ void __launch_bounds__(128, 8) gi_initial_kernel(DevScene s, GiLaunch L, GiImages I) {
     uint32_t x, y;
-    if (!pixel_of(L.cam, x, y)) return;
+    if (!tile_pixel(L.cam, x, y)) return;
     const size_t i = size_t(y) * L.cam.screen_width + x;
     uint32_t seed = make_seed(x, y, L.frame_seed);
     float4 p4, n4;
@@ -123,14 +124,14 @@ __global__ void __launch_bounds__(128, 8) gi_initial_kernel(DevScene s, GiLaunch
         const float3 d = tangent_to_world(sample_cosine_hemisphere(u0, u1, pdf_dir), T, B, pn);
         if (dot(pn, d) <= 0.0f) continue;
         HitRec h;
-        if (!trace<false>(s, make_ray(pp + pn * bias, d), bias, 1e9f, h)) continue;
+        if (!trace_lanes<false, Tree>(s, pp + pn * bias, d, bias, 1e9f, h)) continue;
         const Surface sec = hit_surface(s, h.inst, h.prim, h.u, h.v);
         // evaluate_sample_radiance (:539-552): normal turned toward wo = -d
         const float3 wo = -d;
         float3 sn = sec.normal;
         if (dot(sn, wo) < 0.0f) sn = -sn;
         const Mat sm = load_mat(s, sec.material);
-        const float3 rad = sm.emissive + sample_lights(s, sec.pos, sn, wo, sm, bias, seed);
+        const float3 rad = sm.emissive + sample_lights<Tree>(s, sec.pos, sn, wo, sm, bias, seed);
         const float tgt = gi_target(pp, pn, pm, cp, sec.pos, rad);
         if (tgt <= 0.0f) continue;
         const float pdf = gi_source_pdf(pp, pn, sec.pos);
@@ -371,9 +372,10 @@ __global__ void __launch_bounds__(kBlock) giw_advance_kernel(DevScene s, GiLaunc
 }
 
 // cs_temporal (restir_gi.slang:688-848)
+template <int Tree>
 __global__ void __launch_bounds__(128, 8) gi_temporal_kernel(DevScene s, GiLaunch L, GiImages I) {
     uint32_t x, y;
-    if (!pixel_of(L.cam, x, y)) return;
+    if (!tile_pixel(L.cam, x, y)) return;
     const size_t i = size_t(y) * L.cam.screen_width + x;
     float4 p4, n4;
     float3 pp, pn;
@@ -390,7 +392,7 @@ __global__ void __launch_bounds__(128, 8) gi_temporal_kernel(DevScene s, GiLaunc
     prv.M = min(prv.M, L.m_cap);
     const float jac = reconnection_jacobian(hpos, pp, prv.pos, prv.nrm);
     if (jac <= 0.0f) return;
-    if (!visible(s, pp, pn, prv.pos, L.ray_bias)) return;
+    if (!visible<Tree>(s, pp, pn, prv.pos, L.ray_bias)) return;
     const float ph_prev = gi_target(pp, pn, pm, cp, prv.pos, prv.rad);
     const float contrib = ((ph_prev * mn(prv.W, 50.0f)) * float(prv.M)) * jac;
     if (contrib <= 0.0f) return;
@@ -418,9 +420,10 @@ __global__ void __launch_bounds__(128, 8) gi_temporal_kernel(DevScene s, GiLaunc
 }
 
 // cs_spatial_shade (restir_gi.slang:851-1000)
+template <int Tree>
 __global__ void __launch_bounds__(128, 8) gi_spatial_shade_kernel(DevScene s, GiLaunch L, GiImages I) {
     uint32_t x, y;
-    if (!pixel_of(L.cam, x, y)) return;
+    if (!tile_pixel(L.cam, x, y)) return;
     const uint32_t W = L.cam.screen_width, H = L.cam.screen_height;
     const size_t i = size_t(y) * W + x;
     float3 radiance = f3(0.0f, 0.0f, 0.0f);
@@ -468,7 +471,7 @@ __global__ void __launch_bounds__(128, 8) gi_spatial_shade_kernel(DevScene s, Gi
     }
     if (res.M > 0 && res.W > 0.0f) {
         const float3 ind = gi_indirect(pp, pn, pm, cp, res.pos, res.rad) * res.W;
-        if (luminance(ind) > 0.0f && visible(s, pp, pn, res.pos, L.ray_bias))
+        if (luminance(ind) > 0.0f && visible<Tree>(s, pp, pn, res.pos, L.ray_bias))
             radiance = radiance + ind * L.indirect_strength;
     }
     I.out[i] = make_float4(radiance.x, radiance.y, radiance.z, 1.0f);
@@ -607,7 +610,8 @@ extern "C" rr_status rr_restir_gi_initial(rr_ctx* ctx, const rr_scene* scene, co
     RR_TRY_CUDA(ctx, cudaSetDevice(ctx->device));
     if (ctx->wave_initial && uint64_t(cam->screen_width) * cam->screen_height < (1ull << 31))
         return gi_initial_wavefront(ctx, scene, cam, p, b, static_cast<cudaStream_t>(stream));
-    gi_initial_kernel<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(scene->dev, make_launch(cam, p),
+    const auto kernel = scene->dev.qnodes4 ? gi_initial_kernel<4> : gi_initial_kernel<0>;
+    kernel<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(scene->dev, make_launch(cam, p),
                                                                                   make_images(b));
     RR_CHECK_LAUNCH(ctx);
     ctx->launches += 1;
@@ -622,7 +626,8 @@ extern "C" rr_status rr_restir_gi_temporal(rr_ctx* ctx, const rr_scene* scene, c
     if (st != RR_OK) return st;
     if (!p->temporal_enable) return RR_OK;  // restir_gi.slang:690
     RR_TRY_CUDA(ctx, cudaSetDevice(ctx->device));
-    gi_temporal_kernel<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(scene->dev, make_launch(cam, p),
+    const auto kernel = scene->dev.qnodes4 ? gi_temporal_kernel<4> : gi_temporal_kernel<0>;
+    kernel<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(scene->dev, make_launch(cam, p),
                                                                                    make_images(b));
     RR_CHECK_LAUNCH(ctx);
     ctx->launches += 1;
@@ -636,7 +641,8 @@ extern "C" rr_status rr_restir_gi_spatial_shade(rr_ctx* ctx, const rr_scene* sce
     rr_status st = check(ctx, scene, cam, p, b, kSpatial);
     if (st != RR_OK) return st;
     RR_TRY_CUDA(ctx, cudaSetDevice(ctx->device));
-    gi_spatial_shade_kernel<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    const auto kernel = scene->dev.qnodes4 ? gi_spatial_shade_kernel<4> : gi_spatial_shade_kernel<0>;
+    kernel<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(
         scene->dev, make_launch(cam, p), make_images(b));
     RR_CHECK_LAUNCH(ctx);
     ctx->launches += 1;

@@ -91,9 +91,10 @@ RR_D float target_function(float3 pp, float3 pn, const Mat& pm, float3 cam_pos, 
 }
 
 // cs_initial (restir_pt.slang:567-757)
+template <int Tree>
 __global__ void __launch_bounds__(128, 8) ptr_initial_kernel(DevScene s, PtrLaunch L, PtrImages I) {
     uint32_t x, y;
-    if (!pixel_of(L.cam, x, y)) return;
+    if (!tile_pixel(L.cam, x, y)) return;
     const size_t i = size_t(y) * L.cam.screen_width + x;
     uint32_t seed = make_seed(x, y, L.frame_seed);
     float4 p4, n4;
@@ -121,14 +122,14 @@ __global__ void __launch_bounds__(128, 8) ptr_initial_kernel(DevScene s, PtrLaun
         const float3 wi0 = sample_primary_dir(I.fitted, pp, pn, pmat, L.grid, seed, src_pdf);
         if (src_pdf <= 1e-6f || dot(pn, wi0) <= 0.0f) continue;
         HitRec h;
-        if (!trace<false>(s, make_ray(pp + pn * bias, wi0), bias, 1e9f, h)) continue;
+        if (!trace_lanes<false, Tree>(s, pp + pn * bias, wi0, bias, 1e9f, h)) continue;
         const Surface rc = hit_surface(s, h.inst, h.prim, h.u, h.v);
         float3 rc_n = rc.normal;
         if (dot(rc_n, wi0) > 0.0f) rc_n = -rc_n;
         const Mat rc_mat = load_mat(s, rc.material);
         float3 suffix = rc_mat.emissive;
         const float3 rc_wo = -wi0;
-        suffix = suffix + sample_lights(s, rc.pos, rc_n, rc_wo, rc_mat, bias, seed);
+        suffix = suffix + sample_lights<Tree>(s, rc.pos, rc_n, rc_wo, rc_mat, bias, seed);
         float3 cur_pos = rc.pos, cur_n = rc_n, cur_wo = rc_wo;
         Mat cur_mat = rc_mat;
         float3 path_thp = f3(1.0f, 1.0f, 1.0f);
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(128, 8) ptr_initial_kernel(DevScene s, PtrLaun
             path_thp = path_thp * ((f * cos_at) / pdf);
             if (mx(path_thp.x, mx(path_thp.y, path_thp.z)) <= 0.0f) break;
             HitRec hb;
-            if (!trace<false>(s, make_ray(cur_pos + cur_n * bias, wi), bias, 1e9f, hb)) {
+            if (!trace_lanes<false, Tree>(s, cur_pos + cur_n * bias, wi, bias, 1e9f, hb)) {
                 suffix = suffix + path_thp * sky_radiance(wi);
                 break;
             }
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(128, 8) ptr_initial_kernel(DevScene s, PtrLaun
             if (dot(hn, wi) > 0.0f) hn = -hn;
             const Mat hm = load_mat(s, hs.material);
             const float3 hwo = -wi;
-            suffix = suffix + path_thp * sample_lights(s, hs.pos, hn, hwo, hm, bias, seed);
+            suffix = suffix + path_thp * sample_lights<Tree>(s, hs.pos, hn, hwo, hm, bias, seed);
             cur_pos = hs.pos; cur_n = hn; cur_mat = hm; cur_wo = hwo;
         }
         Reservoir cand;
@@ -480,9 +481,10 @@ __global__ void __launch_bounds__(kBlock) ptrw_advance_kernel(DevScene s, PtrLau
 }
 
 // cs_temporal (restir_pt.slang:760-857)
+template <int Tree>
 __global__ void __launch_bounds__(128, 8) ptr_temporal_kernel(DevScene s, PtrLaunch L, PtrImages I) {
     uint32_t x, y;
-    if (!pixel_of(L.cam, x, y)) return;
+    if (!tile_pixel(L.cam, x, y)) return;
     const uint32_t W = L.cam.screen_width, H = L.cam.screen_height;
     const size_t i = size_t(y) * W + x;
     float4 p4, n4;
@@ -500,7 +502,7 @@ __global__ void __launch_bounds__(128, 8) ptr_temporal_kernel(DevScene s, PtrLau
     prv.M = min(prv.M, L.m_cap);
     const float jac = reconnection_jacobian(hpos, pp, prv.rc_pos, prv.rc_normal);
     if (jac <= 0.0f) return;
-    if (!visible(s, pp, pn, prv.rc_pos, L.ray_bias)) return;
+    if (!visible<Tree>(s, pp, pn, prv.rc_pos, L.ray_bias)) return;
     const float ph_prev = target_function(pp, pn, pm, cp, prv);
     const float prev_W = mn(prv.W, 50.0f);
     const float contrib = ((ph_prev * prev_W) * float(prv.M)) * jac;
@@ -528,9 +530,10 @@ __global__ void __launch_bounds__(128, 8) ptr_temporal_kernel(DevScene s, PtrLau
 }
 
 // cs_spatial_shade (restir_pt.slang:860-1000)
+template <int Tree>
 __global__ void __launch_bounds__(128, 8) ptr_spatial_shade_kernel(DevScene s, PtrLaunch L, PtrImages I) {
     uint32_t x, y;
-    if (!pixel_of(L.cam, x, y)) return;
+    if (!tile_pixel(L.cam, x, y)) return;
     const uint32_t W = L.cam.screen_width, H = L.cam.screen_height;
     const size_t i = size_t(y) * W + x;
     float3 radiance = f3(0.0f, 0.0f, 0.0f);
@@ -579,7 +582,7 @@ __global__ void __launch_bounds__(128, 8) ptr_spatial_shade_kernel(DevScene s, P
     }
     if (res.M > 0 && res.W > 0.0f && res.valid > 0.5f) {
         const float3 ind = evaluate_contribution(pp, pn, pm, cp, res) * res.W;
-        if (luminance(ind) > 0.0f && visible(s, pp, pn, res.rc_pos, L.ray_bias))
+        if (luminance(ind) > 0.0f && visible<Tree>(s, pp, pn, res.rc_pos, L.ray_bias))
             radiance = radiance + ind * L.indirect_strength;
         if (L.grid.enabled != 0u) {  // splat (:978-994)
             const float3 to_rc = res.rc_pos - pp;
@@ -742,7 +745,8 @@ extern "C" rr_status rr_restir_pt_initial(rr_ctx* ctx, const rr_scene* scene, co
     RR_TRY_CUDA(ctx, cudaSetDevice(ctx->device));
     if (ctx->wave_initial && uint64_t(cam->screen_width) * cam->screen_height < (1ull << 31))
         return ptr_initial_wavefront(ctx, scene, cam, p, b, static_cast<cudaStream_t>(stream));
-    ptr_initial_kernel<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(scene->dev, make_launch(cam, p),
+    const auto kernel = scene->dev.qnodes4 ? ptr_initial_kernel<4> : ptr_initial_kernel<0>;
+    kernel<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(scene->dev, make_launch(cam, p),
                                                                                    make_images(b));
     RR_CHECK_LAUNCH(ctx);
     ctx->launches += 1;
@@ -757,7 +761,8 @@ extern "C" rr_status rr_restir_pt_temporal(rr_ctx* ctx, const rr_scene* scene, c
     if (st != RR_OK) return st;
     if (!p->temporal_enable) return RR_OK;  // restir_pt.slang:764
     RR_TRY_CUDA(ctx, cudaSetDevice(ctx->device));
-    ptr_temporal_kernel<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(scene->dev, make_launch(cam, p),
+    const auto kernel = scene->dev.qnodes4 ? ptr_temporal_kernel<4> : ptr_temporal_kernel<0>;
+    kernel<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(scene->dev, make_launch(cam, p),
                                                                                     make_images(b));
     RR_CHECK_LAUNCH(ctx);
     ctx->launches += 1;
@@ -771,7 +776,8 @@ extern "C" rr_status rr_restir_pt_spatial_shade(rr_ctx* ctx, const rr_scene* sce
     rr_status st = check(ctx, scene, cam, p, b, kSpatial);
     if (st != RR_OK) return st;
     RR_TRY_CUDA(ctx, cudaSetDevice(ctx->device));
-    ptr_spatial_shade_kernel<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    const auto kernel = scene->dev.qnodes4 ? ptr_spatial_shade_kernel<4> : ptr_spatial_shade_kernel<0>;
+    kernel<<<grid_of(cam), 128, 0, static_cast<cudaStream_t>(stream)>>>(
         scene->dev, make_launch(cam, p), make_images(b));
     RR_CHECK_LAUNCH(ctx);
     ctx->launches += 1;

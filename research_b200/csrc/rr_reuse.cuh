@@ -83,13 +83,14 @@ RR_D bool sample_light_ray(const DevScene& s, float3 hit_pos, float3 normal, flo
 
 // sample_lights (restir_pt.slang:172-221): one light picked uniformly,
 // shadow ray from hit_pos + normal * ray_bias over [ray_bias, dist - 0.01].
+template <int Tree>
 RR_D float3 sample_lights(const DevScene& s, float3 hit_pos, float3 normal, float3 wo, const Mat& m, float bias,
                           uint32_t& seed) {
     float3 o, d, c;
     float tmax;
     if (!sample_light_ray(s, hit_pos, normal, wo, m, bias, seed, o, d, tmax, c)) return f3(0.0f, 0.0f, 0.0f);
     HitRec h;
-    if (trace<true>(s, make_ray(o, d), bias, tmax, h)) return f3(0.0f, 0.0f, 0.0f);
+    if (trace_lanes<true, Tree>(s, o, d, bias, tmax, h)) return f3(0.0f, 0.0f, 0.0f);
     return c;
 }
 
@@ -106,19 +107,14 @@ RR_D float reconnection_jacobian(float3 src, float3 tgt, float3 rc_pos, float3 r
 }
 
 // trace_visibility (restir_pt.slang:459-469)
+template <int Tree>
 RR_D bool visible(const DevScene& s, float3 origin, float3 normal, float3 target, float bias) {
     const float3 delta = target - origin;
     const float dist = length(delta);
     if (dist <= bias) return false;
     const float3 dir = delta / dist;
     HitRec h;
-    return !trace<true>(s, make_ray(origin + normal * bias, dir), bias, dist - bias, h);
-}
-
-RR_D bool pixel_of(const GpuCameraData& cam, uint32_t& x, uint32_t& y) {
-    x = blockIdx.x * 16 + (threadIdx.x & 15);
-    y = blockIdx.y * 8 + (threadIdx.x >> 4);
-    return x < cam.screen_width && y < cam.screen_height;
+    return !trace_lanes<true, Tree>(s, origin + normal * bias, dir, bias, dist - bias, h);
 }
 
 RR_D float3 cam_pos(const GpuCameraData& c) { return f3(c.position[0], c.position[1], c.position[2]); }

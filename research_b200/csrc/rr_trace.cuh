@@ -234,6 +234,8 @@ struct LocalStackN {
     RR_D E get(int i) const { return e[i]; }
 };
 using LocalStack = LocalStackN<kStackSize>;
+template <bool KeepNear> struct StackEntryOf { using type = int2; };
+template <> struct StackEntryOf<false> { using type = int; };
 template <int S, int Threads, int N = kStackSize, class E = int2>
 struct SplitStack {
     using Entry = E;
@@ -629,6 +631,54 @@ RR_D void quant_leaf(const float4* tris, const QuantRay& q, float tmin, LaneTrav
             }
         }
     } while (++i < end);
+}
+
+// The pixel of a thread in a 16 x 8 pixel block of 128 threads: a warp covers
+// 8 x 4 pixels, so its rays are neighbours in both directions.
+RR_D bool tile_pixel(const GpuCameraData& cam, uint32_t& x, uint32_t& y) {
+    const uint32_t w = threadIdx.x >> 5, l = threadIdx.x & 31u;
+    x = blockIdx.x * 16 + (w & 1u) * 8 + (l & 7u);
+    y = blockIdx.y * 8 + (w >> 1) * 4 + (l >> 3);
+    return x < cam.screen_width && y < cam.screen_height;
+}
+
+// One ray per lane, traced by the lanes that arrive together (any subset of
+// the warp): closest hit, or any hit, in [tmin, tmax]; returns true on hit,
+// `hit` is filled for closest hit. Tree 4: the quantized 4-wide tree with the
+// leaf vote of the queue traversal (rr_wavefront.cuh); a lane that is done
+// waits for the others. Tree 0: trace(), the full-precision tree.
+template <bool AnyHit, int Tree>
+RR_D bool trace_lanes(const DevScene& s, float3 o, float3 d, float tmin, float tmax, HitRec& hit) {
+    if constexpr (Tree == 0) {
+        return trace<AnyHit>(s, make_ray(o, d), tmin, tmax, hit);
+    } else {
+        LocalStackN<kStackSize4, typename StackEntryOf<!AnyHit>::type> stack;
+        const QuantRay r = make_quant_ray(s, o, d);
+        LaneTrav st;
+        lane_begin(st, stack, tmax);
+        const uint32_t lanes = __activemask();
+        while (true) {
+            const uint32_t leafm = __ballot_sync(lanes, st.cur < 0);
+            const uint32_t nodem = __ballot_sync(lanes, st.stepping());
+            if ((leafm | nodem) == 0) break;
+            if (nodem == 0 || __popc(leafm) * 2 > __popc(nodem)) {
+                if (st.cur < 0)
+                    quant_leaf<AnyHit, false>(s.tris, r, tmin, st, nullptr,
+                                              [&](float u, float v, float inst, float prim) {
+                                                  hit.u = u; hit.v = v;
+                                                  hit.inst = __float_as_uint(inst);
+                                                  hit.prim = __float_as_uint(prim);
+                                              });
+            } else {
+                #pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    if (st.stepping()) quant_step4<AnyHit, false>(s.qnodes4, r, tmin, st, stack, nullptr);
+            }
+        }
+        hit.t = st.t;
+        hit.key = st.key;
+        return st.key != kNoIndex;
+    }
 }
 
 // Hit attributes (pathtracer.slang:69-118 / restir_di.slang:108-144):

@@ -104,8 +104,6 @@ __device__ __forceinline__ void flush_work(const TraceWork& w, unsigned long lon
 // SmemS > 0: the bottom SmemS stack entries of every thread in shared memory.
 template <int SmemS, int N, class E> struct QueueStackOf { using type = SplitStack<SmemS, kBlock, N, E>; };
 template <int N, class E> struct QueueStackOf<0, N, E> { using type = LocalStackN<N, E>; };
-template <bool KeepNear> struct QueueEntryOf { using type = int2; };
-template <> struct QueueEntryOf<false> { using type = int; };
 
 constexpr int kNodeSteps = 2;
 constexpr int kBusyLanes = 24;
@@ -116,7 +114,7 @@ __device__ __forceinline__ void traverse_queue(const DevScene& s, const DevScene
                                                Done done, float tmin = 0.001f) {
     TraceWork tw;
     // an any-hit ray's bound never moves: its entries need no distance
-    using Entry = typename QueueEntryOf<Tree == 0 || !AnyHit>::type;
+    using Entry = typename StackEntryOf<Tree == 0 || !AnyHit>::type;
     typename QueueStackOf<SmemS, Tree == 4 ? kStackSize4 : kStackSize, Entry>::type stack;
     if constexpr (SmemS > 0) {
         __shared__ Entry stack_smem[SmemS * kBlock];

@@ -81,3 +81,46 @@ def test_quantized_traversal_bit_exact(rr, O, ctx, torch_cuda, name):
     finally:
         ctx.check(L.rr_pathtracer_set_variants(ctx.handle, 0, 0))
         scene.close()
+
+
+def test_reuse_passes_same_bits_on_both_trees(rr, ctx, torch_cuda):
+    """ReSTIR DI, GI and PT over a scene whose trees are quantized and over
+    the same scene with an instance so far away that they are not (it is last,
+    so the others keep their ids): every image has the same bits. Two frames,
+    an odd image (partial warps at its edges), both forms of the initial
+    passes, DI with and without emitter candidates."""
+    from research_b200 import passes
+    torch = torch_cuda
+    base = rr.HostScene.cornell(0).arrays
+    W, H = 61, 37
+    L = rr.lib()
+    got = []
+    try:
+        for arrays in (base, _outlier(base, 1e7)):
+            scene = rr.Scene(ctx, arrays)
+            images = []
+            for wavefront in (1, 0):
+                ctx.check(L.rr_reuse_set_wavefront(ctx.handle, wavefront))
+                di = passes.ReSTIRDIPass(ctx, (W, H))
+                others = [passes.ReSTIRGIPass(ctx, (W, H)), passes.ReSTIRPTPass(ctx, (W, H))]
+                for k in range(2):
+                    eye = (0.1 * k, 1.0, 3.2)
+                    cam = rr.camera_data(rr.camera_desc(W, H, eye=eye, center=(0.0, 1.0, 0.0)),
+                                         rr.camera_desc(W, H, eye=(0.0, 1.0, 3.2), center=(0.0, 1.0, 0.0)))
+                    di.execute(scene, cam)
+                    images += [di.gbuf_pos.clone(), di.gbuf_norm.clone(), di.output.clone()]
+                    for p in others:
+                        p.execute(scene, cam, di.gbuf_pos, di.gbuf_norm, di.output)
+                        images.append(p.output.clone())
+                z = [torch.zeros((H, W, 4), device="cuda") for _ in range(5)]
+                prm = rr.DIParams(3, 16, 1, 1, 4, 15, 20, rr.DI_FLAG_EMITTERS)
+                ctx.check(L.rr_restir_di_execute(ctx.handle, scene.handle, C.byref(cam), C.byref(prm),
+                                                 *[t.data_ptr() for t in z], torch.cuda.current_stream().cuda_stream))
+                images.append(z[4].clone())
+            got.append([i.cpu().numpy().view(np.uint32) for i in images])
+            scene.close()
+    finally:
+        ctx.check(L.rr_reuse_set_wavefront(ctx.handle, 1))
+    assert got[0][2].any()
+    for k, (a, b) in enumerate(zip(*got)):
+        np.testing.assert_array_equal(a, b, err_msg=f"image {k}")
