@@ -52,6 +52,33 @@ RR_D float3 mul_rows_dir(float4 r0, float4 r1, float4 r2, float3 v) {
               r2.x * v.x + r2.y * v.y + r2.z * v.z);
 }
 
+// ── two FP32 values in one register pair (sm_100's packed instructions:
+// each half rounds as the scalar operation does) and three-operand min / max
+using u64 = unsigned long long;
+RR_D u64 pack2(float a, float b) { u64 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+RR_D float lo2(u64 v) { return __uint_as_float(uint32_t(v)); }
+RR_D float hi2(u64 v) { return __uint_as_float(uint32_t(v >> 32)); }
+RR_D u64 add2(u64 a, u64 b) { u64 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+RR_D u64 fma2(u64 a, u64 b, u64 c) {
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// a * b as a fma with zero: ptxas 12.9 contracts mul.rn.f32x2 and a following
+// add.rn.f32x2 into one fma, which would round once instead of twice. (A
+// negative zero product comes out positive.)
+RR_D u64 mul2(u64 a, u64 b) { return fma2(a, b, 0ull); }
+RR_D float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+RR_D float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 constexpr float kPi = 3.14159265358979323846f;
 constexpr float kTwoPi = 6.28318530717958647692f;
 constexpr float kInvPi = 0.31830988618379067154f;

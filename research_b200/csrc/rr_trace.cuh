@@ -419,25 +419,6 @@ RR_D bool trace4(const DevScene& s, const Ray& r, float tmin, float tmax, HitRec
 // first bounce) and the L1 data path (69 %, node sectors and stack), no
 // longer divergence: 16 of 32 lanes per instruction against 8 with one
 // thread per ray running its leaves' triangle loops inline.
-using u64 = unsigned long long;
-RR_D u64 pack2(float a, float b) { u64 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
-RR_D float lo2(u64 v) { return __uint_as_float(uint32_t(v)); }
-RR_D float hi2(u64 v) { return __uint_as_float(uint32_t(v >> 32)); }
-RR_D u64 fma2(u64 a, u64 b, u64 c) {
-    u64 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-RR_D float max3(float a, float b, float c) {
-    float r;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-RR_D float min3(float a, float b, float c) {
-    float r;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
 RR_D void load32(const void* p, u64& a, u64& b, u64& c, u64& d) {
     asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
 }
@@ -495,6 +476,7 @@ struct LaneTrav {
     int sp;
     float t, tl;       // hit distance so far and the bound boxes are culled with
     uint32_t key;      // the hit triangle's flattened id; kNoIndex: none
+    bool doubtful;     // any hit: at the bound (see quant_leaf)
     RR_D bool stepping() const { return uint32_t(cur) < uint32_t(kDone); }
 };
 
@@ -524,6 +506,7 @@ RR_D void lane_begin(LaneTrav& st, Stack& stack, float tmax) {
     st.t = tmax;
     st.tl = tmax * 1.00001f;
     st.key = kNoIndex;
+    st.doubtful = false;
 }
 
 // The two planes of one axis of a child, as (near, far) distances.
@@ -607,6 +590,13 @@ RR_D void quant_step4(const uint4* nodes, const QuantRay& r, float tmin, LaneTra
 // The triangles of the lane's leaf. Closest hit: the lowest (t, key) is kept
 // and handed to hit(u, v, instance, primitive) (float bits), which every
 // later, nearer one follows; any hit: the first one ends the ray.
+//
+// A hit within a rounding of an any-hit ray's bound is `doubtful`: in the
+// full-precision tree such a triangle is offered only if every inner node
+// above it is entered at near <= tmax (trace_step), which its tight boxes
+// decide by their last bit and the grown ones here do not. That is what rays
+// toward a sample on a surface meet (they end a bias before it), so the
+// caller traces a doubtful ray in the full tree.
 template <bool AnyHit, bool Count, class Hit>
 RR_D void quant_leaf(const float4* tris, const QuantRay& q, float tmin, LaneTrav& st, TraceWork* work, Hit hit) {
     Ray r;
@@ -624,7 +614,7 @@ RR_D void quant_leaf(const float4* tris, const QuantRay& q, float tmin, LaneTrav
         if (intersect_triangle(r, f3(t0.x, t0.y, t0.z), f3(t0.w, t1.x, t1.y), f3(t1.z, t1.w, t2.x), tmin, st.t, tt,
                                uu, vv)) {
             const uint32_t key = __float_as_uint(t2.w);
-            if (AnyHit) { st.key = key; st.cur = kDone; return; }
+            if (AnyHit) { st.key = key; st.doubtful = tt > st.t * 0.999999f; st.cur = kDone; return; }
             if (tt < st.t || key < st.key) {
                 st.t = tt; st.tl = tt * 1.00001f; st.key = key;
                 hit(uu, vv, t2.y, t2.z);
@@ -640,6 +630,17 @@ RR_D bool tile_pixel(const GpuCameraData& cam, uint32_t& x, uint32_t& y) {
     x = blockIdx.x * 16 + (w & 1u) * 8 + (l & 7u);
     y = blockIdx.y * 8 + (w >> 1) * 4 + (l >> 3);
     return x < cam.screen_width && y < cam.screen_height;
+}
+
+// trace() in the full-precision tree, out of line: for the few doubtful rays.
+template <bool AnyHit>
+__device__ __noinline__ bool trace_full(const float4* nodes, const float4* tris, uint32_t num_nodes, float3 o, float3 d,
+                                        float tmin, float tmax, HitRec* hit) {
+    DevScene s{};
+    s.nodes = nodes;
+    s.tris = tris;
+    s.num_nodes = num_nodes;
+    return trace<AnyHit>(s, make_ray(o, d), tmin, tmax, *hit);
 }
 
 // One ray per lane, traced by the lanes that arrive together (any subset of
@@ -675,6 +676,7 @@ RR_D bool trace_lanes(const DevScene& s, float3 o, float3 d, float tmin, float t
                     if (st.stepping()) quant_step4<AnyHit, false>(s.qnodes4, r, tmin, st, stack, nullptr);
             }
         }
+        if (AnyHit && st.doubtful) return trace_full<AnyHit>(s.nodes, s.tris, s.num_nodes, o, d, tmin, tmax, &hit);
         hit.t = st.t;
         hit.key = st.key;
         return st.key != kNoIndex;

@@ -153,16 +153,29 @@ __device__ __forceinline__ void traverse_queue(const DevScene& s, const DevScene
         st.cur = kFree;
         uint32_t i = 0;
         bool more = true;   // the queue may hold entries not taken yet
+        // Doubtful any-hit rays (quant_leaf), traced in the full tree at the
+        // end; a warp that holds 32 of them leaves its share of the queue to
+        // the loop there.
+        __shared__ uint32_t doubt_smem[AnyHit ? kBlock / 32 : 1][AnyHit ? 64 : 1];
+        uint32_t* const doubt = doubt_smem[AnyHit ? threadIdx.x >> 5 : 0];
+        uint32_t doubts = 0;
         while (true) {
             const uint32_t leafm = __ballot_sync(kFull, st.cur < 0);
             const uint32_t nodem = __ballot_sync(kFull, st.stepping());
-            if ((leafm | nodem) == 0 || (more && __popc(leafm | nodem) <= kBusyLanes)) {
+            const bool take = more && (!AnyHit || doubts < 32u);
+            if ((leafm | nodem) == 0 || (take && __popc(leafm | nodem) <= kBusyLanes)) {
                 const bool idle = st.cur >= kDone;
+                const bool doubtful = AnyHit && st.cur == kDone && st.doubtful;
                 if (st.cur == kDone) {
-                    done(i, st.key != kNoIndex);
+                    if (!doubtful) done(i, st.key != kNoIndex);
                     st.cur = kFree;
                 }
-                if (!more) break;   // nobody is busy
+                if constexpr (AnyHit) {
+                    const uint32_t m = __ballot_sync(kFull, doubtful);
+                    if (doubtful) doubt[doubts + __popc(m & ((1u << lane_id()) - 1u))] = i;
+                    doubts += __popc(m);
+                }
+                if (!take) break;   // nobody is busy
                 const uint32_t idlem = __ballot_sync(kFull, idle);
                 uint32_t base = 0;
                 if (lane_id() == 0) base = atomicAdd(cursor, __popc(idlem));
@@ -198,6 +211,25 @@ __device__ __forceinline__ void traverse_queue(const DevScene& s, const DevScene
                         if constexpr (Tree == 4) quant_step4<AnyHit, Count>(nodes, r, tmin, st, stack, &tw);
                         else quant_step2<AnyHit, Count>(nodes, r, tmin, st, stack, &tw);
                     }
+            }
+        }
+        if constexpr (AnyHit) {
+            auto trace_one = [&](uint32_t e) {
+                float3 o, d;
+                float tmax;
+                const uint32_t sid = load(e, o, d, tmax);
+                const DevScene& es = Multi ? table[sid] : s;
+                HitRec h;
+                done(e, trace<true, Count>(es, make_ray(o, d), tmin, tmax, h, &tw));
+            };
+            __syncwarp();
+            for (uint32_t k = lane_id(); k < doubts; k += 32u) trace_one(doubt[k]);
+            while (more) {
+                uint32_t base = 0;
+                if (lane_id() == 0) base = atomicAdd(cursor, 32u);
+                base = __shfl_sync(kFull, base, 0);
+                more = base < count;
+                if (base + lane_id() < count) trace_one(base + lane_id());
             }
         }
     }

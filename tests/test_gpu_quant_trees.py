@@ -124,3 +124,72 @@ def test_reuse_passes_same_bits_on_both_trees(rr, ctx, torch_cuda):
     assert got[0][2].any()
     for k, (a, b) in enumerate(zip(*got)):
         np.testing.assert_array_equal(a, b, err_msg=f"image {k}")
+
+
+def test_visibility_at_the_far_bound_matches_the_full_tree(rr, ctx, torch_cuda):
+    """Shadow rays that meet a surface at their far bound, within a rounding:
+    from the floor straight up to samples on the ceiling and on the light
+    below it (the ray starts a bias above the floor and ends a bias before the
+    sample). Which of them count as blocked follows the full-precision tree's
+    rule, so ReSTIR GI's shading agrees with rr_trace_counted ray by ray."""
+    torch = torch_cuda
+    L = rr.lib()
+    st = torch.cuda.current_stream().cuda_stream
+    scene = rr.Scene(ctx, rr.HostScene.cornell(0).arrays)
+    W = H = 256
+    g = torch.Generator(device="cuda").manual_seed(7)
+    r = lambda: torch.rand((H, W), device="cuda", generator=g)
+    img = lambda *c: torch.stack(list(c), -1).contiguous()
+    one, zero = torch.ones((H, W), device="cuda"), torch.zeros((H, W), device="cuda")
+    px, pz = (r() - 0.5) * 1.6, (r() - 0.5) * 1.6
+    # up to a tenth of the height off the vertical
+    tx, tz = px + (r() - 0.5) * 0.1 * r(), pz + (r() - 0.5) * 0.1 * r()
+    ty = torch.where((tx.abs() < 0.25) & (tz.abs() < 0.25), torch.tensor(0.999, device="cuda"), one)
+    # the floor's material index: any non-emissive one
+    mats = rr.HostScene.cornell(0).arrays["materials"]
+    mat = int(np.nonzero(mats["emissive"].max(1) == 0)[0][0])
+    bits = torch.full((H, W), mat, dtype=torch.int32, device="cuda").view(torch.float32)
+    gpos, gnrm = img(px, zero, pz, one), img(zero, one, zero, bits)
+    m1 = torch.full((H, W), 1, dtype=torch.int32, device="cuda").view(torch.float32)
+    res = [img(tx, ty, tz, one), img(one, one, one, one), img(zero, -one, zero, m1)]
+    spare = [torch.zeros((H, W, 4), device="cuda") for _ in range(8)]
+    im = rr.GiReuseImages()
+    im.gbuf_pos, im.gbuf_norm, im.direct = gpos.data_ptr(), gnrm.data_ptr(), None
+    for k in range(3):
+        im.reservoir_curr[k], im.reservoir_prev[k] = res[k].data_ptr(), spare[k].data_ptr()
+    for k in range(2):
+        im.history_curr[k], im.history_prev[k] = spare[3 + k].data_ptr(), spare[5 + k].data_ptr()
+    im.output = spare[7].data_ptr()
+    bias = 1e-3
+    p = rr.gi_reuse_params(1, 8, 0, 0, 0, 12, 0, 1.0, bias)
+    cam = rr.camera_data(rr.camera_desc(W, H, eye=(0.0, 0.5, 3.2), center=(0.0, 0.5, 0.0)))
+    ctx.check(L.rr_restir_gi_spatial_shade(ctx.handle, scene.handle, C.byref(cam), C.byref(p), C.byref(im), st))
+    lit = spare[7][..., :3].amax(-1) > 0
+    # the same rays, operation by operation
+    dx, dy, dz = tx - px, ty - zero, tz - pz
+    xx, yy, zz = dx * dx, dy * dy, dz * dz
+    dist = ((xx + yy) + zz).sqrt()
+    b = torch.tensor(bias, device="cuda")
+    origins = img(px + zero * b, zero + one * b, pz + zero * b, zero).view(-1, 4)
+    dirs = img(dx / dist, dy / dist, dz / dist, zero).view(-1, 4)
+    tmax = (dist - b).view(-1)
+    n = W * H
+    hits, prims = torch.empty((n, 4), device="cuda"), torch.empty(n, device="cuda", dtype=torch.int32)
+    work = torch.empty((n, 2), device="cuda", dtype=torch.int32)
+    blocked = torch.zeros(n, dtype=torch.bool, device="cuda")
+    # rr_trace_counted takes one tmax a call: one call per distinct value near the bound, so group by value
+    order = tmax.argsort()
+    values, counts = torch.unique_consecutive(tmax[order], return_counts=True)
+    first = 0
+    for v, c in list(zip(values.tolist(), counts.tolist()))[:4000]:
+        o, d = origins[order[first:first + c]].contiguous(), dirs[order[first:first + c]].contiguous()
+        ctx.check(L.rr_trace_counted(ctx.handle, scene.handle, o.data_ptr(), d.data_ptr(), bias, v, c, rr.TRACE_ANY_HIT,
+                                     hits.data_ptr(), prims.data_ptr(), work.data_ptr(), st))
+        blocked[order[first:first + c]] = hits[:c, 0] >= 0
+        first += c
+    done = order[:first]
+    got = lit.view(-1)[done]
+    want = ~blocked[done]
+    assert first > 1000 and 0 < int(want.sum()) < first
+    assert int((got != want).sum()) == 0
+    scene.close()
