@@ -328,9 +328,10 @@ rr_status rr_atrous_execute(rr_ctx* ctx, const float* input, const float* gbuf_p
                             const float* gbuf_norm, float* ping0, float* ping1,
                             const rr_atrous_params* params, uint32_t* out_slot, void* stream);
 
-/* Strides 1, 2 and 4 run a kernel whose blocks first copy their halo tile
- * of the three images into shared memory with TMA tensor copies (default
- * on; the same bits as the direct-load kernel, which strides 8 and up use).
+/* A stride whose lattice fills 32 x 16 tiles runs a kernel that filters a
+ * tile of it in shared memory. At stride 1 the tile is copied there with TMA
+ * tensor copies (default on; the same bits with plain loads, which the other
+ * strides use).
  * A block whose copies miss the kernel's bounded wait (wait_tries tries,
  * default 2^22) sets a host-mapped flag, waits once more (bounded) for its
  * copies, and filters its pixels from global memory instead: the output is
