@@ -140,10 +140,10 @@ __global__ void __launch_bounds__(kBlock, 4) guided_shade_kernel(DevScene s0, Gu
                                                               const uint32_t* count_ptr,
                                                               uint32_t* next_count, uint32_t* shadow_count) {
     const uint32_t count = *count_ptr;
-    const uint32_t warp_first = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = warp_first; base < count; base += stride) {
-        const uint32_t i = base + lane_id();
+    __shared__ AllocTable<2> table_smem;
+    uint32_t turn = 0;
+    for (uint32_t base = blockIdx.x * kBlock; base < count; base += gridDim.x * kBlock, ++turn) {
+        const uint32_t i = base + threadIdx.x;
         bool cont = false, emit_shadow = false;
         uint32_t pid = 0, seed = 0, sid = 0;
         float3 new_o = f3(0, 0, 0), wi = f3(0, 0, 0), thp = f3(0, 0, 0);
@@ -347,13 +347,16 @@ __global__ void __launch_bounds__(kBlock, 4) guided_shade_kernel(DevScene s0, Gu
             }
         }
         const float tag = Multi ? __uint_as_float(sid) : 0.0f;
-        const uint32_t sslot = warp_alloc(emit_shadow, shadow_count);
+        const bool want[2] = {emit_shadow, cont};
+        uint32_t* const counters[2] = {shadow_count, next_count};
+        uint32_t slot[2];
+        block_alloc(table_smem, turn, want, counters, slot);
+        const uint32_t sslot = slot[0], rslot = slot[1];
         if (emit_shadow) {
             sa[sslot] = make_float4(sh_o.x, sh_o.y, sh_o.z, __uint_as_float(pid));
             sb[sslot] = make_float4(sh_d.x, sh_d.y, sh_d.z, sh_tmax);
             sc[sslot] = make_float4(contrib.x, contrib.y, contrib.z, tag);
         }
-        const uint32_t rslot = warp_alloc(cont, next_count);
         if (cont) {
             na[rslot] = make_float4(new_o.x, new_o.y, new_o.z, __uint_as_float(pid));
             nb[rslot] = make_float4(wi.x, wi.y, wi.z, __uint_as_float(seed));
@@ -1272,7 +1275,7 @@ static rr_status enqueue_guided_batch(rr_ctx* ctx, rr_batch* B, rr_guide* const*
     {
         const uint64_t threads = uint64_t(tiles) * 32;
         raygen_batch_kernel<<<uint32_t((threads + kBlock - 1) / kBlock), kBlock, 0, stream>>>(
-            entries, count, tiles, outs, q.ray_a[0], q.ray_b[0], q.ray_c[0], C);
+            entries, count, tiles, uint32_t(paths), outs, q.ray_a[0], q.ray_b[0], q.ray_c[0], C);
         RR_CHECK_LAUNCH(ctx);
         launches += 1;
     }

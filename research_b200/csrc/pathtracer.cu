@@ -304,10 +304,10 @@ __global__ void __launch_bounds__(kBlock, 4) shade_kernel(DevScene s, const DevS
                                                        const uint32_t* count_ptr,
                                                        uint32_t* next_count, uint32_t* shadow_count) {
     const uint32_t count = *count_ptr;
-    const uint32_t warp_first = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = warp_first; base < count; base += stride) {
-        const uint32_t i = base + lane_id();
+    __shared__ AllocTable<2> table_smem;
+    uint32_t turn = 0;
+    for (uint32_t base = blockIdx.x * kBlock; base < count; base += gridDim.x * kBlock, ++turn) {
+        const uint32_t i = base + threadIdx.x;
         ShadeResult R;
         uint32_t sid = 0;
         if (i < count) {
@@ -323,13 +323,16 @@ __global__ void __launch_bounds__(kBlock, 4) shade_kernel(DevScene s, const DevS
             }
         }
         const float tag = Multi ? __uint_as_float(sid) : 0.0f;
-        const uint32_t sslot = warp_alloc(R.emit_shadow, shadow_count);
+        const bool want[2] = {R.emit_shadow, R.cont};
+        uint32_t* const counters[2] = {shadow_count, next_count};
+        uint32_t slot[2];
+        block_alloc(table_smem, turn, want, counters, slot);
+        const uint32_t sslot = slot[0], rslot = slot[1];
         if (R.emit_shadow) {
             sa[sslot] = make_float4(R.sh_o.x, R.sh_o.y, R.sh_o.z, __uint_as_float(R.pid));
             sb[sslot] = make_float4(R.sh_d.x, R.sh_d.y, R.sh_d.z, R.sh_tmax);
             sc[sslot] = make_float4(R.contrib.x, R.contrib.y, R.contrib.z, tag);
         }
-        const uint32_t rslot = warp_alloc(R.cont, next_count);
         if (R.cont) {
             na[rslot] = make_float4(R.new_o.x, R.new_o.y, R.new_o.z, __uint_as_float(R.pid));
             nb[rslot] = make_float4(R.wi.x, R.wi.y, R.wi.z, __uint_as_float(R.seed));
@@ -547,7 +550,7 @@ rr_status enqueue_batch(rr_ctx* ctx, rr_batch* B, uint32_t total_tiles, size_t n
         rr_stage_timer t0(ctx, stream, timed);
         t0.begin(0);
         raygen_batch_kernel<<<uint32_t((threads + kBlock - 1) / kBlock), kBlock, 0, stream>>>(
-            entries, count_scenes, total_tiles, outs, q.ray_a[0], q.ray_b[0], q.ray_c[0], C);
+            entries, count_scenes, total_tiles, uint32_t(n), outs, q.ray_a[0], q.ray_b[0], q.ray_c[0], C);
         RR_CHECK_LAUNCH(ctx);
         t0.end(0);
         rr_status st0 = t0.commit();
@@ -684,6 +687,7 @@ rr_status rr_batch_stage_call(rr_ctx* ctx, rr_batch* B, const GpuCameraData* cam
         e.L.tiles_x = (c.screen_width + 7) / 8;
         e.L.tiles_per_image = e.L.tiles_x * ((c.screen_height + 3) / 4);
         e.tile_begin = tiles;
+        e.path_begin = uint32_t(paths);
         const uint64_t t = uint64_t(e.L.tiles_per_image) * p->spp;
         if (uint64_t(tiles) + t >= (1ull << 26))
             return rr_fail(ctx, RR_ERR_INVALID_ARGUMENT, "rr_batch_execute: too many tiles");

@@ -223,14 +223,18 @@ RR_D void giw_finish(const GiLaunch& L, const GiImages& I, const GiWave& V, size
 }
 
 __global__ void __launch_bounds__(kBlock) giw_begin_kernel(DevScene s, GiLaunch L, GiImages I, GiWave V) {
-    const uint32_t W = L.cam.screen_width;
-    const uint32_t warp_first = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
-    for (uint32_t base = warp_first; base < V.n; base += gridDim.x * blockDim.x) {
-        const uint32_t i = base + lane_id();
+    // a warp takes an 8 x 4 pixel tile, so that its rays are neighbours
+    const uint32_t W = L.cam.screen_width, H = L.cam.screen_height;
+    const uint32_t tiles_x = (W + 7u) / 8u, threads = tiles_x * ((H + 3u) / 4u) * 32u;
+    __shared__ AllocTable<1> table_smem;
+    uint32_t turn = 0;
+    for (uint32_t base = blockIdx.x * kBlock; base < threads; base += gridDim.x * kBlock, ++turn) {
+        const uint32_t tile = (base + threadIdx.x) >> 5;
+        const uint32_t x = tile % tiles_x * 8u + (lane_id() & 7u), y = tile / tiles_x * 4u + (lane_id() >> 3);
+        const uint32_t i = y * W + x;
         bool emit = false;
         float3 o = f3(0.0f, 0.0f, 0.0f), d = f3(0.0f, 0.0f, 0.0f);
-        if (i < V.n) {
-            const uint32_t x = i % W, y = i / W;
+        if (x < W && y < H) {
             uint32_t seed = make_seed(x, y, L.frame_seed);
             float4 p4, n4;
             float3 pp, pn;
@@ -254,10 +258,13 @@ __global__ void __launch_bounds__(kBlock) giw_begin_kernel(DevScene s, GiLaunch 
                 }
             }
         }
-        const uint32_t slot = warp_alloc(emit, V.cnt);
+        const bool want[1] = {emit};
+        uint32_t* const counters[1] = {V.cnt};
+        uint32_t slot[1];
+        block_alloc(table_smem, turn, want, counters, slot);
         if (emit) {
-            V.qa[0][slot] = make_float4(o.x, o.y, o.z, __uint_as_float(i));
-            V.qb[0][slot] = make_float4(d.x, d.y, d.z, 0.0f);
+            V.qa[0][slot[0]] = make_float4(o.x, o.y, o.z, __uint_as_float(i));
+            V.qb[0][slot[0]] = make_float4(d.x, d.y, d.z, 0.0f);
         }
     }
 }
@@ -267,9 +274,10 @@ __global__ void __launch_bounds__(kBlock, 4) giw_shade_kernel(DevScene s, GiLaun
     uint32_t* c0 = V.cnt + size_t(step) * kWaveWords;
     const uint32_t count = c0[0];
     const float bias = L.ray_bias;
-    const uint32_t warp_first = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
-    for (uint32_t base = warp_first; base < count; base += gridDim.x * blockDim.x) {
-        const uint32_t q = base + lane_id();
+    __shared__ AllocTable<2> table_smem;
+    uint32_t turn = 0;
+    for (uint32_t base = blockIdx.x * kBlock; base < count; base += gridDim.x * kBlock, ++turn) {
+        const uint32_t q = base + threadIdx.x;
         bool shadow = false, ris = false;
         uint32_t pid = 0;
         float3 so = f3(0.0f, 0.0f, 0.0f), sd = so, sc = so;
@@ -301,14 +309,17 @@ __global__ void __launch_bounds__(kBlock, 4) giw_shade_kernel(DevScene s, GiLaun
                 ris = true;
             }
         }
-        const uint32_t sslot = warp_alloc(shadow, c0 + 2);
+        // every segment ends its candidate (a miss drops it)
+        const bool want[2] = {shadow, q < count};
+        uint32_t* const counters[2] = {c0 + 2, c0 + 4};
+        uint32_t slot[2];
+        block_alloc(table_smem, turn, want, counters, slot);
+        const uint32_t sslot = slot[0], eslot = slot[1];
         if (shadow) {
             V.sa[sslot] = make_float4(so.x, so.y, so.z, __uint_as_float(pid));
             V.sb[sslot] = make_float4(sd.x, sd.y, sd.z, stmax);
             V.sc[sslot] = make_float4(sc.x, sc.y, sc.z, 0.0f);
         }
-        // every segment ends its candidate (a miss drops it)
-        const uint32_t eslot = warp_alloc(q < count, c0 + 4);
         if (q < count) V.ended[eslot] = pid | (ris ? kRis : 0u);
     }
 }
@@ -320,9 +331,10 @@ __global__ void __launch_bounds__(kBlock) giw_advance_kernel(DevScene s, GiLaunc
     uint32_t* c1 = c0 + kWaveWords;
     const uint32_t count = c0[4];
     const float3 cp = cam_pos(L.cam);
-    const uint32_t warp_first = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
-    for (uint32_t base = warp_first; base < count; base += gridDim.x * blockDim.x) {
-        const uint32_t q = base + lane_id();
+    __shared__ AllocTable<1> table_smem;
+    uint32_t turn = 0;
+    for (uint32_t base = blockIdx.x * kBlock; base < count; base += gridDim.x * kBlock, ++turn) {
+        const uint32_t q = base + threadIdx.x;
         bool emit = false;
         uint32_t pid = 0;
         float3 o = f3(0.0f, 0.0f, 0.0f), d = o;
@@ -363,10 +375,13 @@ __global__ void __launch_bounds__(kBlock) giw_advance_kernel(DevScene s, GiLaunc
                 giw_finish(L, I, V, pid, pp, pn, pm, M_count, w_sum);
             }
         }
-        const uint32_t slot = warp_alloc(emit, c1);
+        const bool want[1] = {emit};
+        uint32_t* const counters[1] = {c1};
+        uint32_t slot[1];
+        block_alloc(table_smem, turn, want, counters, slot);
         if (emit) {
-            V.qa[nxt][slot] = make_float4(o.x, o.y, o.z, __uint_as_float(pid));
-            V.qb[nxt][slot] = make_float4(d.x, d.y, d.z, 0.0f);
+            V.qa[nxt][slot[0]] = make_float4(o.x, o.y, o.z, __uint_as_float(pid));
+            V.qb[nxt][slot[0]] = make_float4(d.x, d.y, d.z, 0.0f);
         }
     }
 }
