@@ -7,7 +7,7 @@
 //   shade  : miss/sky and emissive termination (:213-229), NEE light pick and
 //            shadow-ray emission (:124-177), BSDF sample, throughput update,
 //            Russian roulette (:236-260); survivors are compacted into the
-//            next ray queue with one warp ballot + one atomic per warp
+//            next ray queue with one atomic per block
 //   shadow : any-hit traversal; unoccluded NEE contributions are added
 // The RNG state travels with each ray, so every path consumes random numbers
 // in the reference order (primary 2, per bounce NEE 1 -> BSDF 2 -> RR 1).
