@@ -20,10 +20,10 @@
 //    features, N=out, K=128 samples) on the tensor cores, then
 //    dZ_{l-1} = dX_l * [X_l > 0] in place in shared memory; dW_0^T last.
 //    X_l and dZ_4 arrive by tensor copies (TMA); every CTA accumulates its
-//    tiles' weight gradients in TMEM and writes one FP32 partial;
-//    mlp_reduce_kernel sums the partials in CTA order.
-//  - mlp_adam_kernel: Adam on FP32 master weights and biases (gradients carry
-//    a static loss scale), refreshing the BF16 copy used by the tensor cores;
+//    tiles' weight gradients in TMEM and writes one FP32 partial.
+//  - mlp_update_kernel: the partials' sum in CTA order, then Adam on FP32
+//    master weights and biases (gradients carry a static loss scale),
+//    refreshing the BF16 copy used by the tensor cores;
 //    the forward kernel adds the biases inside the MMA (a constant-1 input
 //    column against a BF16 bias column of the weight tile).
 
@@ -281,7 +281,8 @@ struct FwdArgs {
     const double* wnorm;          // [0] = clamp value, [1] = 1 / (sum of clamped weights)
     __nv_bfloat16* X;             // [batch][kXCols], inputs of every layer
     __nv_bfloat16* dZ;            // [batch][kZCols], the forward writes the output layer's block
-    float* loss_partial;          // per block
+    float* loss_partial;          // per block, zero for the blocks not launched
+    uint32_t loss_parts;
     // grouped inference: group g's rows are slots group_base[g] + [0, group_count[g]) of surf/mix,
     // its tiles [tile_prefix[g], tile_prefix[g + 1]), its network nets[g]
     const MlpView* nets;
@@ -523,6 +524,8 @@ __global__ void __launch_bounds__(kTile * NW, Grouped ? 3 : 1) mlp_forward_kerne
             __syncthreads();
         }
         if (threadIdx.x == 0) A.loss_partial[blockIdx.x] = red[0];
+        if (blockIdx.x == 0)
+            for (uint32_t i = gridDim.x + threadIdx.x; i < A.loss_parts; i += blockDim.x) A.loss_partial[i] = 0.0f;
     }
     if (!ok && t == 0 && V.error) atomicExch(V.error, 1);
     tc::fence_before_sync();
@@ -778,23 +781,30 @@ __global__ void __maxnreg__(128) mlp_backward_kernel(const __grid_constant__ CUt
     }
 }
 
-// grad = sum of the CTA partials in CTA order.
-__global__ void __launch_bounds__(256) mlp_reduce_kernel(const float* __restrict__ partial, uint32_t parts,
-                                                         float* __restrict__ grad) {
+// grad = sum of the CTA partials in CTA order, then the Adam step. Bound by
+// the 148 loads' latency: sixteen at a time, and one launch for both (14 us as
+// a sum with the compiler's unrolling and a launch for the step).
+constexpr int kUpdateThreads = 128;
+__global__ void __launch_bounds__(kUpdateThreads) mlp_update_kernel(const float* __restrict__ partial, uint32_t parts,
+                                                                    float* __restrict__ grad,
+                                                                    float* __restrict__ params, float* __restrict__ m,
+                                                                    float* __restrict__ v,
+                                                                    __nv_bfloat16* __restrict__ w16, float lr,
+                                                                    float bc1, float bc2) {
+    constexpr uint32_t kAhead = 16;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= kParams) return;
     float s = 0.0f;
-    for (uint32_t c = 0; c < parts; ++c) s += partial[size_t(c) * kParams + p];
+    for (uint32_t c0 = 0; c0 < parts; c0 += kAhead) {
+        float q[kAhead];
+        #pragma unroll
+        for (uint32_t u = 0; u < kAhead; ++u) q[u] = c0 + u < parts ? partial[size_t(c0 + u) * kParams + p] : 0.0f;
+        #pragma unroll
+        for (uint32_t u = 0; u < kAhead; ++u)
+            if (c0 + u < parts) s += q[u];
+    }
     grad[p] = s;
-}
-
-__global__ void __launch_bounds__(256) mlp_adam_kernel(float* __restrict__ params, const float* __restrict__ grad,
-                                                       float* __restrict__ m, float* __restrict__ v,
-                                                       __nv_bfloat16* __restrict__ w16, float lr, float bc1,
-                                                       float bc2) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kParams) return;
-    const float g = grad[p] / kLossScale;
+    const float g = s / kLossScale;
     const float mm = 0.9f * m[p] + 0.1f * g;
     const float vv = 0.999f * v[p] + 0.001f * g * g;
     m[p] = mm;
@@ -808,48 +818,69 @@ __global__ void __launch_bounds__(256) mlp_adam_kernel(float* __restrict__ param
 
 // Batch weight normalisation (clamp = 20 x mean, then 1 / sum of clamped
 // weights), as two fixed-order reductions: block b sums the batch slice
-// [b n / G, (b+1) n / G) in FP64, then one warp adds the G partials in a
-// fixed order.
+// [b n / G, (b+1) n / G) in FP64, then one warp of the block that finishes
+// last adds the G partials in a fixed order (lane l partials l, l + 32, ...,
+// then a butterfly). The first pass also selects the batch: element i is
+// sample (i n / batch + offset) mod n. Bound by latency: a thread's loads
+// (seven for a batch of 2^18) are in flight together. (The selection, the
+// two sums and their finishes as launches of their own: 30 us for 2^18.)
 constexpr int kWnBlocks = 148;
-__global__ void __launch_bounds__(256) mlp_wsum_kernel(GuideSamples S, const uint32_t* __restrict__ sel, uint32_t n,
-                                                       const double* __restrict__ wnorm, bool clamped,
-                                                       double* __restrict__ partial) {
+template <bool First>
+__global__ void __launch_bounds__(256) mlp_wsum_kernel(const float4* __restrict__ s0, uint32_t* __restrict__ sel,
+                                                       uint32_t batch, uint32_t n, uint32_t offset,
+                                                       double* __restrict__ wnorm, double* __restrict__ partial,
+                                                       uint32_t* __restrict__ ticket) {
+    constexpr uint32_t kAhead = 8;
     __shared__ double red[256];
+    __shared__ bool last;
     const int t = threadIdx.x;
-    const uint32_t b0 = uint32_t((uint64_t(blockIdx.x) * n) / gridDim.x);
-    const uint32_t b1 = uint32_t((uint64_t(blockIdx.x + 1) * n) / gridDim.x);
-    const double cv = clamped ? wnorm[0] : 0.0;
+    const uint32_t b0 = uint32_t((uint64_t(blockIdx.x) * batch) / gridDim.x);
+    const uint32_t b1 = uint32_t((uint64_t(blockIdx.x + 1) * batch) / gridDim.x);
+    const double cv = First ? 0.0 : wnorm[0];
     double s = 0.0;
-    for (uint32_t i = b0 + t; i < b1; i += 256) {
-        const double w = double(S.s0[sel[i]].w);
-        s += clamped ? fmin(w, cv) : w;
+    for (uint32_t i0 = b0 + t; i0 < b1; i0 += kAhead * 256) {
+        float w[kAhead];
+        #pragma unroll
+        for (uint32_t u = 0; u < kAhead; ++u) {
+            const uint32_t i = i0 + u * 256;
+            w[u] = 0.0f;
+            if (i < b1) {
+                uint32_t k;
+                if (First) sel[i] = k = uint32_t((uint64_t(i) * n) / batch + offset) % n;
+                else k = sel[i];
+                w[u] = s0[k].w;
+            }
+        }
+        #pragma unroll
+        for (uint32_t u = 0; u < kAhead; ++u)
+            if (i0 + u * 256 < b1) s += First ? double(w[u]) : fmin(double(w[u]), cv);
     }
     red[t] = s;
     __syncthreads();
-    for (int k = 128; k > 0; k >>= 1) {
+    for (int k = 128; k > 16; k >>= 1) {
         if (t < k) red[t] += red[t + k];
         __syncthreads();
     }
-    if (t == 0) partial[blockIdx.x] = red[0];
-}
-
-// One warp: lane l adds partials l, l + 32, ... in order, then the lanes'
-// sums are combined by a fixed butterfly (the same order every run).
-__global__ void __launch_bounds__(32) mlp_wfinish_kernel(const double* __restrict__ partial, uint32_t parts,
-                                                         uint32_t n, bool clamped, double* __restrict__ wnorm) {
-    double s = 0.0;
-    for (uint32_t c = threadIdx.x; c < parts; c += 32) s += partial[c];
+    if (t < 32) {
+        s = red[t];
+        #pragma unroll
+        for (int k = 16; k > 0; k >>= 1) s += __shfl_down_sync(0xffffffffu, s, k);
+    }
+    if (t == 0) {
+        partial[blockIdx.x] = s;
+        __threadfence();
+        last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;   // back to 0 for the next launch
+    }
+    __syncthreads();
+    if (!last || t >= 32) return;
+    __threadfence();
+    s = 0.0;
+    for (uint32_t c = t; c < gridDim.x; c += 32) s += __ldcg(partial + c);
     #pragma unroll
     for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (threadIdx.x != 0) return;
-    if (!clamped) wnorm[0] = 20.0 * (s / double(n > 0 ? n : 1));
+    if (t != 0) return;
+    if (First) wnorm[0] = 20.0 * (s / double(batch > 0 ? batch : 1));
     else wnorm[1] = s > 0.0 ? 1.0 / s : 0.0;
-}
-
-__global__ void mlp_select_kernel(uint32_t* sel, uint32_t batch, uint32_t n, uint32_t offset) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= batch) return;
-    sel[i] = uint32_t((uint64_t(i) * n) / batch + offset) % n;
 }
 
 // deterministic uniform init (hash), He-uniform for hidden layers
@@ -888,6 +919,7 @@ struct rr_mlp_state {
     float* loss_partial = nullptr;
     float* wpartial = nullptr;    // per backward CTA: kParams FP32
     double* wn_partial = nullptr; // per weight-norm block
+    uint32_t* wn_ticket = nullptr;
     int wg_grid = 0;
     uint32_t batch_cap = 0;
     uint32_t steps = 0;
@@ -944,6 +976,8 @@ rr_status rr_mlp_guide_init(rr_ctx* ctx, rr_guide* g) {
     M.wg_grid = ctx->sm_count;
     if ((st = al(reinterpret_cast<void**>(&M.wpartial), size_t(M.wg_grid) * kParams * 4)) != RR_OK) return st;
     if ((st = al(reinterpret_cast<void**>(&M.wn_partial), size_t(kWnBlocks) * 8)) != RR_OK) return st;
+    if ((st = al(reinterpret_cast<void**>(&M.wn_ticket), 4)) != RR_OK) return st;
+    RR_TRY_CUDA(ctx, cudaMemset(M.wn_ticket, 0, 4));
     RR_TRY_CUDA(ctx, cudaMallocHost(&M.loss_host, size_t(M.grid) * 4));
     RR_TRY_CUDA(ctx, cudaFuncSetAttribute(mlp_forward_kernel<true, false, kTrainWG>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, fwd_smem(kTrainWG)));
@@ -1067,12 +1101,11 @@ rr_status rr_mlp_guide_train(rr_ctx* ctx, rr_guide* g, uint32_t n, cudaStream_t 
     rr_mlp_state& M = *g->mlp;
     if (n == 0) return RR_OK;
     const uint32_t B = std::min(n, M.batch_cap);
-    mlp_select_kernel<<<(B + 255) / 256, 256, 0, stream>>>(M.sel, B, n, (M.steps * 7919u) % n);
-    RR_CHECK_LAUNCH(ctx);
-    mlp_wsum_kernel<<<kWnBlocks, 256, 0, stream>>>(g->samples, M.sel, B, M.wnorm, false, M.wn_partial);
-    mlp_wfinish_kernel<<<1, 32, 0, stream>>>(M.wn_partial, kWnBlocks, B, false, M.wnorm);
-    mlp_wsum_kernel<<<kWnBlocks, 256, 0, stream>>>(g->samples, M.sel, B, M.wnorm, true, M.wn_partial);
-    mlp_wfinish_kernel<<<1, 32, 0, stream>>>(M.wn_partial, kWnBlocks, B, true, M.wnorm);
+    const uint32_t offset = (M.steps * 7919u) % n;
+    mlp_wsum_kernel<true><<<kWnBlocks, 256, 0, stream>>>(g->samples.s0, M.sel, B, n, offset, M.wnorm, M.wn_partial,
+                                                         M.wn_ticket);
+    mlp_wsum_kernel<false><<<kWnBlocks, 256, 0, stream>>>(g->samples.s0, M.sel, B, n, offset, M.wnorm, M.wn_partial,
+                                                          M.wn_ticket);
     RR_CHECK_LAUNCH(ctx);
     FwdArgs A{};
     A.V = rr_mlp_guide_view(g);
@@ -1083,9 +1116,9 @@ rr_status rr_mlp_guide_train(rr_ctx* ctx, rr_guide* g, uint32_t n, cudaStream_t 
     A.X = M.X;
     A.dZ = M.dZ;
     A.loss_partial = M.loss_partial;
+    A.loss_parts = uint32_t(M.grid);
     const uint32_t tiles = (B + kTile - 1) / kTile;
     const int fgrid = int(std::min<uint32_t>((tiles + kTrainWG - 1) / kTrainWG, uint32_t(ctx->sm_count)));
-    RR_TRY_CUDA(ctx, cudaMemsetAsync(M.loss_partial, 0, size_t(M.grid) * 4, stream));
     mlp_forward_kernel<true, false, kTrainWG><<<fgrid, kTile * kTrainWG, fwd_smem(kTrainWG), stream>>>(A);
     RR_CHECK_LAUNCH(ctx);
     // The backward's copies are boxes of kTile rows; a batch of fewer rows
@@ -1106,16 +1139,14 @@ rr_status rr_mlp_guide_train(rr_ctx* ctx, rr_guide* g, uint32_t n, cudaStream_t 
     const int bgrid = int(std::min<uint32_t>((tiles + kBwdWG - 1) / kBwdWG, uint32_t(M.wg_grid)));
     mlp_backward_kernel<<<bgrid, kTile * kBwdWG, kBwdSmem, stream>>>(mx, mz, Bw);
     RR_CHECK_LAUNCH(ctx);
-    mlp_reduce_kernel<<<(kParams + 255) / 256, 256, 0, stream>>>(M.wpartial, uint32_t(bgrid), M.grad);
-    RR_CHECK_LAUNCH(ctx);
     M.steps += 1;
     const float bc1 = 1.0f - std::pow(0.9f, float(M.steps));
     const float bc2 = 1.0f - std::pow(0.999f, float(M.steps));
-    mlp_adam_kernel<<<(kParams + 255) / 256, 256, 0, stream>>>(M.params, M.grad, M.adam_m, M.adam_v, M.w16,
-                                                               g->desc.learning_rate, bc1, bc2);
+    mlp_update_kernel<<<(kParams + kUpdateThreads - 1) / kUpdateThreads, kUpdateThreads, 0, stream>>>(
+        M.wpartial, uint32_t(bgrid), M.grad, M.params, M.adam_m, M.adam_v, M.w16, g->desc.learning_rate, bc1, bc2);
     RR_CHECK_LAUNCH(ctx);
     RR_TRY_CUDA(ctx, cudaMemcpyAsync(M.loss_host, M.loss_partial, size_t(M.grid) * 4, cudaMemcpyDeviceToHost, stream));
-    ctx->launches += 10;
+    ctx->launches += 5;
     return RR_OK;
 }
 
