@@ -397,8 +397,10 @@ extern "C" rr_status rr_pathtracer_execute(rr_ctx* ctx, const rr_scene* scene,
     const bool emitters = (p->flags & RR_PT_FLAG_EMITTERS) != 0;
     using ShadeKernel = decltype(&shade_kernel<false, false>);
     const ShadeKernel shade_k = emitters ? shade_kernel<false, true> : shade_kernel<false, false>;
-    const int g_shade = std::min<int>(persistent_grid(ctx, reinterpret_cast<const void*>(shade_k)),
-                                      int((n + kBlock - 1) / kBlock));
+    // a block per 256 paths, handed to the SMs as they finish: 16.28 against
+    // 16.34 ms for the 1080p frame with a resident grid (batches and guided
+    // frames, of fewer paths, gain nothing from it)
+    const int g_shade = int((n + kBlock - 1) / kBlock);
     if (count) RR_TRY_CUDA(ctx, cudaMemsetAsync(ctx->work64, 0, sizeof(unsigned long long) * 4, stream));
     const DevScene& S = scene->dev;
     float4* out = reinterpret_cast<float4*>(radiance_out);

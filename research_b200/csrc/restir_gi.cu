@@ -344,13 +344,15 @@ __global__ void __launch_bounds__(kBlock) giw_advance_kernel(DevScene s, GiLaunc
             const uint4 st = V.st[pid];
             uint32_t seed = st.x, c = st.y, M_count = st.w;
             float w_sum = V.acc[pid].x;
+            // the candidate's loads go out with the surface's, whether it enters
+            // resampling or not
+            const float3 spos = xyz(V.spos[pid]), rad = xyz(V.rad[pid]);
             float4 p4, n4;
             float3 pp, pn;
             uint32_t pmat;
             load_surface(s, I.gpos, I.gnrm, pid, p4, n4, pp, pn, pmat);
             const Mat pm = load_mat(s, pmat);
             if (e & kRis) {
-                const float3 spos = xyz(V.spos[pid]), rad = xyz(V.rad[pid]);
                 const float tgt = gi_target(pp, pn, pm, cp, spos, rad);
                 if (!(tgt <= 0.0f)) {
                     const float pdf = gi_source_pdf(pp, pn, spos);
