@@ -986,7 +986,8 @@ extern "C" rr_status rr_guided_pathtracer_execute(rr_ctx* ctx, const rr_scene* s
         uint32_t* cn = C + 4 * (b + 1);
         G.bounce = b;
         G.last = b + 1 == p->max_bounces ? 1u : 0u;
-        ext_k<<<g_ext, kBlock, 0, stream>>>(S, q.ray_a[cur], q.ray_b[cur], q.hits, cb, cb + 1, ctx->work64);
+        ext_k<<<g_ext, kBlock, 0, stream>>>(S, q.ray_a[cur], q.ray_b[cur], q.hits, cb, cb + 1, ctx->work64,
+                                            refill_of(b));
         RR_CHECK_LAUNCH(ctx);
         if (mlp && !G.last) {
             guided_surface_kernel<<<g_shade, kBlock, 0, stream>>>(S, q.ray_b[cur], q.hits, g->mlp_surf, cb);
@@ -1308,7 +1309,7 @@ static rr_status enqueue_guided_batch(rr_ctx* ctx, rr_batch* B, rr_guide* const*
         G.bounce = b;
         G.last = b + 1 == max_bounces ? 1u : 0u;
         ext_k<<<g_ext, kBlock, 0, stream>>>(B->d_table, q.ray_a[cur], q.ray_b[cur], q.ray_c[cur], q.hits, cb, cb + 1,
-                                            ctx->work64);
+                                            ctx->work64, refill_of(b));
         RR_CHECK_LAUNCH(ctx);
         if (mlp && !G.last) {
             RR_TRY_CUDA(ctx, cudaMemsetAsync(B->group_count, 0, sizeof(uint32_t) * count, stream));

@@ -417,7 +417,8 @@ extern "C" rr_status rr_pathtracer_execute(rr_ctx* ctx, const rr_scene* scene,
         uint32_t* cb = C + 4 * b;
         uint32_t* cn = C + 4 * (b + 1);
         timer.begin(1);
-        ext_k<<<g_ext, kBlock, 0, stream>>>(S, q.ray_a[cur], q.ray_b[cur], q.hits, cb, cb + 1, ctx->work64);
+        ext_k<<<g_ext, kBlock, 0, stream>>>(S, q.ray_a[cur], q.ray_b[cur], q.hits, cb, cb + 1, ctx->work64,
+                                            refill_of(b));
         RR_CHECK_LAUNCH(ctx);
         timer.end(1);
         if (overlap && b > 0) RR_TRY_CUDA(ctx, cudaStreamWaitEvent(stream, ctx->shadowed[b - 1], 0));
@@ -581,7 +582,7 @@ rr_status enqueue_batch(rr_ctx* ctx, rr_batch* B, uint32_t total_tiles, size_t n
         uint32_t* cn = C + 4 * (b + 1);
         timer.begin(1);
         ext_k<<<g_ext, kBlock, 0, stream>>>(B->d_table, q.ray_a[cur], q.ray_b[cur], q.ray_c[cur], q.hits, cb, cb + 1,
-                                            ctx->work64);
+                                            ctx->work64, refill_of(b));
         RR_CHECK_LAUNCH(ctx);
         timer.end(1);
         if (overlap && b > 0) RR_TRY_CUDA(ctx, cudaStreamWaitEvent(stream, ctx->shadowed[b - 1], 0));

@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(kBlock, 4) wave_extend_kernel(DevScene s, cons
             tmax = 1e9f;
             return 0u;
         },
-        StoreHit{hits}, StoreMiss{hits}, tmin);
+        StoreHit{hits}, StoreMiss{hits}, kBusyLanes, tmin);
 }
 
 template <int Tree, int SmemS>
@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(kBlock, 4) wave_shadow_kernel(DevScene s, cons
             const float3 v = xyz(sum[pid]) + add;
             sum[pid] = make_float4(v.x, v.y, v.z, 0.0f);
         },
-        tmin);
+        kBusyLanes, tmin);
 }
 
 using WaveExtendKernel = decltype(&wave_extend_kernel<4, 12>);

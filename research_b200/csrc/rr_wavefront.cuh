@@ -135,15 +135,20 @@ __device__ __forceinline__ void flush_work(const TraceWork& w, unsigned long lon
 //     on its own would idle the other 31 for some 100 instructions per
 //     triangle: that took two thirds of the issue slots);
 //   rays: idle lanes finish their rays and take the queue's next entries,
-//     once at most kBusyLanes are busy (neighbouring entries are neighbouring
-//     paths after compaction, so rays stay alike).
+//     once at most `refill` are busy (neighbouring entries are neighbouring
+//     paths after compaction, so rays stay alike). That is kBusyLanes, but 0
+//     for camera rays: a warp's 32 cross the same nodes as long as all are
+//     from one tile (1.92 ms for the 1080p frame's 8.3 M; refilled at 8, 16,
+//     24 busy lanes 2.06 / 2.33 / 2.35. The first bounce's rays take 3.91 /
+//     3.45 / 3.34 / 3.19, and shadow rays 2.91 / 2.50 / 2.18 / 2.07).
 // Measured on the 1080p 4 spp frame of the 1M-triangle room, extension /
 // shadow rays: one thread per ray 16.6 / 11.8 ms; this loop on the
 // full-precision tree, leaf vote 1/4, 1/2, 1: 14.4 / 14.2 / 14.4 and 10.1 /
 // 9.8 / 10.0 ms; with refill at 8, 16, 24 busy lanes 13.8 / 13.7 / 13.4 and
 // 8.8 / 8.1 / 7.8 ms; on the quantized binary tree 12.5 / 6.9 ms; leaves as
 // references and one, two, three node steps a vote 11.5 / 10.8 / 10.5 and
-// 6.4 / 6.1 / 5.8 ms; 4-wide, two steps, stack in shared memory 9.4 / 5.1 ms.
+// 6.4 / 6.1 / 5.8 ms; 4-wide, two steps, stack in shared memory 9.3 / 5.2 ms;
+// camera rays without refill 8.9 ms.
 //
 // Tree 0: the binary tree in full precision, one thread per ray (scenes that
 // the grid does not serve).
@@ -153,12 +158,12 @@ template <int SmemS, int N, class E> struct QueueStackOf { using type = SplitSta
 template <int N, class E> struct QueueStackOf<0, N, E> { using type = LocalStackN<N, E>; };
 
 constexpr int kNodeSteps = 2;
-constexpr int kBusyLanes = 24;
+constexpr uint32_t kBusyLanes = 24;
 
 template <bool AnyHit, bool Count, bool Multi, int Tree, int SmemS, class Load, class Hit, class Done>
 __device__ __forceinline__ void traverse_queue(const DevScene& s, const DevScene* __restrict__ table, uint32_t count,
                                                uint32_t* cursor, unsigned long long* work_out, Load load, Hit hit,
-                                               Done done, float tmin = 0.001f) {
+                                               Done done, uint32_t refill, float tmin = 0.001f) {
     TraceWork tw;
     // an any-hit ray's bound never moves: its entries need no distance
     using Entry = typename StackEntryOf<Tree == 0 || !AnyHit>::type;
@@ -210,7 +215,7 @@ __device__ __forceinline__ void traverse_queue(const DevScene& s, const DevScene
             const uint32_t leafm = __ballot_sync(kFull, st.cur < 0);
             const uint32_t nodem = __ballot_sync(kFull, st.stepping());
             const bool take = more && (!AnyHit || doubts < 32u);
-            if ((leafm | nodem) == 0 || (take && __popc(leafm | nodem) <= kBusyLanes)) {
+            if ((leafm | nodem) == 0 || (take && uint32_t(__popc(leafm | nodem)) <= refill)) {
                 const bool idle = st.cur >= kDone;
                 const bool doubtful = AnyHit && st.cur == kDone && st.doubtful;
                 if (st.cur == kDone) {
@@ -306,7 +311,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) extend_kernel(DevScene s, c
                                                                    const float4* __restrict__ qb,
                                                                    float4* __restrict__ hits,
                                                                    const uint32_t* count_ptr, uint32_t* cursor,
-                                                                   unsigned long long* work_out) {
+                                                                   unsigned long long* work_out, uint32_t refill) {
     traverse_queue<false, Count, false, Tree, SmemS>(
         s, nullptr, *count_ptr, cursor, work_out,
         [&](uint32_t i, float3& o, float3& d, float& tmax) -> uint32_t {
@@ -315,7 +320,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) extend_kernel(DevScene s, c
             tmax = 1e9f;
             return 0u;
         },
-        StoreHit{hits}, StoreMiss{hits});
+        StoreHit{hits}, StoreMiss{hits}, refill);
 }
 
 // Any-hit shadow rays; unoccluded NEE contributions are added to the image.
@@ -344,7 +349,8 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) shadow_kernel(DevScene s, c
                 o.x = o.x + c.x; o.y = o.y + c.y; o.z = o.z + c.z;
                 out[pid] = o;
             }
-        });
+        },
+        kBusyLanes);
 }
 
 // ── batches of scenes (no reference counterpart: the reference renders one
@@ -409,7 +415,8 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) extend_batch_kernel(const D
                                                                          const float4* __restrict__ qc,
                                                                          float4* __restrict__ hits,
                                                                          const uint32_t* count_ptr, uint32_t* cursor,
-                                                                         unsigned long long* work_out) {
+                                                                         unsigned long long* work_out,
+                                                                         uint32_t refill) {
     const DevScene none{};
     traverse_queue<false, Count, true, Tree, SmemS>(
         none, table, *count_ptr, cursor, work_out,
@@ -419,7 +426,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) extend_batch_kernel(const D
             tmax = 1e9f;
             return __float_as_uint(qc[i].w);
         },
-        StoreHit{hits}, StoreMiss{hits});
+        StoreHit{hits}, StoreMiss{hits}, refill);
 }
 
 template <bool Count, int MinBlocks, int Tree, int SmemS>
@@ -450,19 +457,21 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) shadow_batch_kernel(const D
                 o.x = o.x + c.x; o.y = o.y + c.y; o.z = o.z + c.z;
                 out[pid] = o;
             }
-        });
+        },
+        kBusyLanes);
 }
 
 using BatchQueueKernel = void (*)(const DevScene*, const float4*, const float4*, const float4*, float4*,
-                                  const uint32_t*, uint32_t*, unsigned long long*);
+                                  const uint32_t*, uint32_t*, unsigned long long*, uint32_t);
 using BatchShadowKernel = void (*)(const DevScene*, float4* const*, const float4*, const float4*, const float4*,
                                    const uint32_t*, uint32_t*, unsigned long long*);
 // Traversal kernel variants (rr_pathtracer_set_variants): MinBlocks x tree x
 // stack entries in shared memory. A scene whose trees are not quantized is
 // traced by kVariantFull's kernel whatever the variant. kVariantDefault is
 // the fastest on the 1M-triangle room (extension / shadow rays of the 1080p
-// frame 9.4 / 5.1 ms; 9.5 / 5.3 ms with the whole stack in local memory;
-// binary tree 10.4 / 5.5 ms).
+// frame 8.9 / 5.2 ms; with camera rays refilled 9.3, 9.5 / 5.3 with the
+// whole stack in local memory,
+// binary tree 10.4 / 5.5).
 constexpr int kVariantFull = 7, kVariantDefault = 4;
 #define RR_TRAVERSAL_VARIANTS(kernel, v)                   \
     switch (v) {                                           \
@@ -482,13 +491,16 @@ template <bool Count>
 BatchShadowKernel shadow_batch_variant(int v) { RR_TRAVERSAL_VARIANTS(shadow_batch_kernel, v) }
 
 using QueueKernel = void (*)(DevScene, const float4*, const float4*, float4*, const uint32_t*, uint32_t*,
-                             unsigned long long*);
+                             unsigned long long*, uint32_t);
 using ShadowKernel = void (*)(DevScene, const float4*, const float4*, const float4*, float4*, const uint32_t*,
                               uint32_t*, unsigned long long*);
 template <bool Count>
 QueueKernel extend_variant(int v) { RR_TRAVERSAL_VARIANTS(extend_kernel, v) }
 template <bool Count>
 ShadowKernel shadow_variant(int v) { RR_TRAVERSAL_VARIANTS(shadow_kernel, v) }
+
+// When a bounce's extension rays are refilled (traverse_queue).
+uint32_t refill_of(uint32_t bounce) { return bounce == 0 ? 0u : kBusyLanes; }
 
 // The variant a scene's rays run: the asked one, or the full-precision form.
 int variant_for(const DevScene& s, int v) { return s.qnodes4 ? v : kVariantFull; }
