@@ -566,7 +566,7 @@ def run_ours(args, ws, rank, local):
                         "source": "ncu capture of one frame's extend launches, summarised in "
                                   "profiles/extend_traffic.txt; not measured in this run"}
     roofline = {"kernel": "extend_kernel (closest-hit BVH traversal, all bounces of one frame)",
-                "bound": "latency (L1/L2-served node fetches, SIMT divergence)",
+                "bound": "instruction issue (box tests at half the lanes), L1/L2 latency of node fetches",
                 "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_kind": f"{peak_kind} hbm_gbs", "traffic": None, "from_profile": from_profile,
                 "achieved_scope": "algorithmic bytes (rays, BVH nodes and triangles the traversal touches, counted by "

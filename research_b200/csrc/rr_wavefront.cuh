@@ -469,9 +469,8 @@ using BatchShadowKernel = void (*)(const DevScene*, float4* const*, const float4
 // stack entries in shared memory. A scene whose trees are not quantized is
 // traced by kVariantFull's kernel whatever the variant. kVariantDefault is
 // the fastest on the 1M-triangle room (extension / shadow rays of the 1080p
-// frame 8.9 / 5.2 ms; with camera rays refilled 9.3, 9.5 / 5.3 with the
-// whole stack in local memory,
-// binary tree 10.4 / 5.5).
+// frame 8.9 / 5.2 ms; 9.1 / 5.2 with the whole stack in local memory,
+// binary tree 9.9 / 6.0).
 constexpr int kVariantFull = 7, kVariantDefault = 4;
 #define RR_TRAVERSAL_VARIANTS(kernel, v)                   \
     switch (v) {                                           \
