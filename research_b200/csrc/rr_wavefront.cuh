@@ -159,6 +159,8 @@ template <int N, class E> struct QueueStackOf<0, N, E> { using type = LocalStack
 
 constexpr int kNodeSteps = 2;
 constexpr uint32_t kBusyLanes = 24;
+constexpr uint32_t kDoubtList = 64, kDoubtStop = 32;   // a warp's list of doubtful rays (traverse_queue)
+static_assert(kDoubtStop - 1 + 32 <= kDoubtList, "the list holds a warp's rays on top of those it stops at");
 
 template <bool AnyHit, bool Count, bool Multi, int Tree, int SmemS, class Load, class Hit, class Done>
 __device__ __forceinline__ void traverse_queue(const DevScene& s, const DevScene* __restrict__ table, uint32_t count,
@@ -206,15 +208,17 @@ __device__ __forceinline__ void traverse_queue(const DevScene& s, const DevScene
         uint32_t i = 0;
         bool more = true;   // the queue may hold entries not taken yet
         // Doubtful any-hit rays (quant_leaf), traced in the full tree at the
-        // end; a warp that holds 32 of them leaves its share of the queue to
-        // the loop there.
-        __shared__ uint32_t doubt_smem[AnyHit ? kBlock / 32 : 1][AnyHit ? 64 : 1];
+        // end; a warp that holds kDoubtStop of them leaves its share of the
+        // queue to the loop there. Rays are taken only while fewer are listed,
+        // the turn's own included, so each of the 32 lanes' rays still has a
+        // place if all of them turn out doubtful.
+        __shared__ uint32_t doubt_smem[AnyHit ? kBlock / 32 : 1][AnyHit ? kDoubtList : 1];
         uint32_t* const doubt = doubt_smem[AnyHit ? threadIdx.x >> 5 : 0];
         uint32_t doubts = 0;
         while (true) {
             const uint32_t leafm = __ballot_sync(kFull, st.cur < 0);
             const uint32_t nodem = __ballot_sync(kFull, st.stepping());
-            const bool take = more && (!AnyHit || doubts < 32u);
+            bool take = more && (!AnyHit || doubts < kDoubtStop);
             if ((leafm | nodem) == 0 || (take && uint32_t(__popc(leafm | nodem)) <= refill)) {
                 const bool idle = st.cur >= kDone;
                 const bool doubtful = AnyHit && st.cur == kDone && st.doubtful;
@@ -226,8 +230,12 @@ __device__ __forceinline__ void traverse_queue(const DevScene& s, const DevScene
                     const uint32_t m = __ballot_sync(kFull, doubtful);
                     if (doubtful) doubt[doubts + __popc(m & ((1u << lane_id()) - 1u))] = i;
                     doubts += __popc(m);
+                    take = more && doubts < kDoubtStop;
                 }
-                if (!take) break;   // nobody is busy
+                if (!take) {
+                    if ((leafm | nodem) == 0) break;
+                    continue;   // the busy lanes go on
+                }
                 const uint32_t idlem = __ballot_sync(kFull, idle);
                 uint32_t base = 0;
                 if (lane_id() == 0) base = atomicAdd(cursor, __popc(idlem));
