@@ -31,6 +31,7 @@ struct DevScene {
     const uint4* qnodes;      // both trees with quantized boxes (see QuantRay), or null
     const uint4* qnodes4;
     float3 qbase, qscale;     // grid plane q of an axis: qbase + (128 + q / 256) * qscale
+    float3 qinv;              // 1 / qscale
     const float4* vertices;   // GpuVertex as 3 float4
     const uint32_t* indices;
     const uint4* meshes;      // GpuMesh as 2 uint4
@@ -426,14 +427,16 @@ RR_D void load32(const void* p, u64& a, u64& b, u64& c, u64& d) {
 // A ray against the grid. Plane q reads as f = 128 + q / 256 (its 15 bits put
 // into a float's mantissa by one byte permute, whose selector picks the near
 // or the far plane by the direction's sign), and t(q) = f * s + off with s =
-// qscale / d and off = (qbase - o) / d -/+ m. Rounding: s is off by u (2^-24)
-// relative, at most 256 u |s| in t; qbase - o, its product with 1/d and the
-// sum with m by u each, 3 u |qbase - o| / |d|, and the far side's factor once
-// more each; m = 8 u (|qbase - o| + 128 qscale) / |d| is more than all of these, so near planes only move nearer
-// and far ones farther. What is left is relative (the fma, 1/d), and covered
-// by the factor 1.000002 on the far side and 1.00001 on the hit bound, as in
-// box_pair. px..pz keep the shear axes in their upper halves, which the
-// permute does not read.
+// qscale * inv and off = (qbase - o) * inv -/+ m (inv: make_ray's, the same in
+// both trees). m is such that every near distance comes out no farther, and
+// every far one no nearer, than box_pair's of the box that the grid box was
+// grown from: a box box_pair opens is opened here too. With u = 2^-24 and C =
+// |qbase - o|, and everything times |inv|: the slopes are off by at most 512 u
+// qscale, the offsets by 5 u C, the sum by u (256 qscale + C); box_pair's own
+// planes are up to 6.1 u |o| (its offsets) and 2 u (256 qscale + C) away
+// from exact. Together less than m = 8 u (C + |o| + 192 qscale).
+// px..pz keep the shear axes in their upper halves, which the permute does
+// not read.
 struct QuantRay {
     u64 sx, sy, sz;        // (near, far) slopes
     u64 ox, oy, oz;        // (near, far) offsets
@@ -450,7 +453,7 @@ RR_D QuantRay make_quant_ray(const DevScene& sc, float3 o, float3 d) {
     auto axis = [](float org, float inv, float base, float scale, u64& s, u64& off, uint32_t& p, uint32_t& f) {
         const float c = base - org;
         const float a = c * inv;
-        const float m = 4.76837158203125e-7f * fabsf(inv) * (fabsf(c) + 128.0f * scale);
+        const float m = 4.76837158203125e-7f * fabsf(inv) * (fabsf(c) + fabsf(org) + 192.0f * scale);
         const float k = scale * inv;
         s = pack2(k, k * 1.000002f);
         off = pack2(a - m, (a + m) * 1.000002f);
@@ -475,8 +478,7 @@ struct LaneTrav {
     int cur;
     int sp;
     float t, tl;       // hit distance so far and the bound boxes are culled with
-    uint32_t key;      // the hit triangle's flattened id; kNoIndex: none
-    bool doubtful;     // any hit: at the bound (see quant_leaf)
+    uint32_t tri;      // the hit triangle's place in the leaves' order; kNoIndex: none
     RR_D bool stepping() const { return uint32_t(cur) < uint32_t(kDone); }
 };
 
@@ -505,8 +507,7 @@ RR_D void lane_begin(LaneTrav& st, Stack& stack, float tmax) {
     st.cur = 0;
     st.t = tmax;
     st.tl = tmax * 1.00001f;
-    st.key = kNoIndex;
-    st.doubtful = false;
+    st.tri = kNoIndex;
 }
 
 // The two planes of one axis of a child, as (near, far) distances.
@@ -589,14 +590,8 @@ RR_D void quant_step4(const uint4* nodes, const QuantRay& r, float tmin, LaneTra
 
 // The triangles of the lane's leaf. Closest hit: the lowest (t, key) is kept
 // and handed to hit(u, v, instance, primitive) (float bits), which every
-// later, nearer one follows; any hit: the first one ends the ray.
-//
-// A hit within a rounding of an any-hit ray's bound is `doubtful`: in the
-// full-precision tree such a triangle is offered only if every inner node
-// above it is entered at near <= tmax (trace_step), which its tight boxes
-// decide by their last bit and the grown ones here do not. That is what rays
-// toward a sample on a surface meet (they end a bias before it), so the
-// caller traces a doubtful ray in the full tree.
+// later, nearer one follows; any hit: the first one ends the ray. The hit
+// stands only if in_own_box says so.
 template <bool AnyHit, bool Count, class Hit>
 RR_D void quant_leaf(const float4* tris, const QuantRay& q, float tmin, LaneTrav& st, TraceWork* work, Hit hit) {
     Ray r;
@@ -613,14 +608,49 @@ RR_D void quant_leaf(const float4* tris, const QuantRay& q, float tmin, LaneTrav
         float tt, uu, vv;
         if (intersect_triangle(r, f3(t0.x, t0.y, t0.z), f3(t0.w, t1.x, t1.y), f3(t1.z, t1.w, t2.x), tmin, st.t, tt,
                                uu, vv)) {
-            const uint32_t key = __float_as_uint(t2.w);
-            if (AnyHit) { st.key = key; st.doubtful = tt > st.t * 0.999999f; st.cur = kDone; return; }
-            if (tt < st.t || key < st.key) {
-                st.t = tt; st.tl = tt * 1.00001f; st.key = key;
+            if (AnyHit) { st.tri = uint32_t(i); st.cur = kDone; return; }
+            if (tt < st.t || st.tri == kNoIndex ||
+                __float_as_uint(t2.w) < __float_as_uint(__ldg(tris + size_t(st.tri) * 3 + 2).w)) {
+                st.t = tt; st.tl = tt * 1.00001f; st.tri = uint32_t(i);
                 hit(uu, vv, t2.y, t2.z);
             }
         }
     } while (++i < end);
+}
+
+// Whether the full-precision tree is certain to offer a ray the triangle
+// (place i) that it hit through the grown boxes: box_pair's test of the
+// triangle's own box, which every box above it contains. (The planes' distances
+// are monotone, so those boxes pass if it does.) The triangle test's distance
+// is rounded by a few u times the triangle's size, and the tight boxes are what
+// keeps such a distance from counting where the ray does not cross the
+// triangle: the floor a ray leaves (one of triangles of 4e4 is hit again at
+// 1e-3), a needle's plane, a surface that an any-hit ray ends before.
+// limit: tmax for any hit, up to which inner nodes are entered (trace_step), and
+// 1.00001 t for a closest one. With true for a hit, and nothing hit through the
+// larger boxes for a miss, an any-hit answer is the full tree's. So is a
+// closest hit, unless another surface lies within that 1e-5 of it: there the
+// lowest (t, key) is kept, which the full tree may pass over (1 of 10^8 rays, on
+// edges that two triangles share). A ray whose hit fails is doubtful: it is
+// traced in the full tree.
+//
+// 1/d is the slope over the grid's step, 3 u off; a distance is 5 u off then,
+// where box_pair's are at most 2 u on the other side of exact. The factors 1 +
+// 10 u (near) and 1 + 20 u (far, 1.000002 in box_pair) make up for that, so
+// a box that passes here passes there. It costs the 1080p frame 0.57 ms (15.73
+// to 16.31): half the triangle's loads and this arithmetic, half the loop that
+// traces the doubtful rays. (0.74 ms with the ray reloaded and its divisions.)
+RR_D bool in_own_box(const float4* tris, uint32_t i, const QuantRay& r, float3 qinv, float tmin, float limit) {
+    const float4 t0 = __ldg(tris + size_t(i) * 3 + 0);
+    const float4 t1 = __ldg(tris + size_t(i) * 3 + 1);
+    const float4 t2 = __ldg(tris + size_t(i) * 3 + 2);
+    const float ix = lo2(r.sx) * qinv.x, iy = lo2(r.sy) * qinv.y, iz = lo2(r.sz) * qinv.z;
+    const float tx0 = (min3(t0.x, t0.w, t1.z) - r.o.x) * ix, tx1 = (max3(t0.x, t0.w, t1.z) - r.o.x) * ix;
+    const float ty0 = (min3(t0.y, t1.x, t1.w) - r.o.y) * iy, ty1 = (max3(t0.y, t1.x, t1.w) - r.o.y) * iy;
+    const float tz0 = (min3(t0.z, t1.y, t2.x) - r.o.z) * iz, tz1 = (max3(t0.z, t1.y, t2.x) - r.o.z) * iz;
+    const float near = fmaxf(max3(fminf(tx0, tx1), fminf(ty0, ty1), fminf(tz0, tz1)) * 1.0000006f, tmin);
+    const float far = min3(fmaxf(tx0, tx1), fmaxf(ty0, ty1), fmaxf(tz0, tz1)) * 1.0000012f;
+    return near <= fminf(far, limit);
 }
 
 // The pixel of a thread in a 16 x 8 pixel block of 128 threads: a warp covers
@@ -676,10 +706,11 @@ RR_D bool trace_lanes(const DevScene& s, float3 o, float3 d, float tmin, float t
                     if (st.stepping()) quant_step4<AnyHit, false>(s.qnodes4, r, tmin, st, stack, nullptr);
             }
         }
-        if (AnyHit && st.doubtful) return trace_full<AnyHit>(s.nodes, s.tris, s.num_nodes, o, d, tmin, tmax, &hit);
+        if (st.tri == kNoIndex) return false;
+        if (!in_own_box(s.tris, st.tri, r, s.qinv, tmin, AnyHit ? tmax : st.tl))
+            return trace_full<AnyHit>(s.nodes, s.tris, s.num_nodes, o, d, tmin, tmax, &hit);
         hit.t = st.t;
-        hit.key = st.key;
-        return st.key != kNoIndex;
+        return true;
     }
 }
 

@@ -202,36 +202,37 @@ __device__ __forceinline__ void traverse_queue(const DevScene& s, const DevScene
     } else {
         const uint4* nodes = Tree == 4 ? s.qnodes4 : s.qnodes;
         const float4* tris = s.tris;
+        float3 qinv = s.qinv;
         QuantRay r;
         LaneTrav st;
         st.cur = kFree;
         uint32_t i = 0;
         bool more = true;   // the queue may hold entries not taken yet
-        // Doubtful any-hit rays (quant_leaf), traced in the full tree at the
-        // end; a warp that holds kDoubtStop of them leaves its share of the
-        // queue to the loop there. Rays are taken only while fewer are listed,
-        // the turn's own included, so each of the 32 lanes' rays still has a
-        // place if all of them turn out doubtful.
-        __shared__ uint32_t doubt_smem[AnyHit ? kBlock / 32 : 1][AnyHit ? kDoubtList : 1];
-        uint32_t* const doubt = doubt_smem[AnyHit ? threadIdx.x >> 5 : 0];
+        // Doubtful rays (in_own_box), traced in the full tree at the end; a
+        // warp that holds kDoubtStop of them leaves its share of the queue to
+        // the loop there. Rays are taken only while fewer are listed, the
+        // turn's own included, so each of the 32 lanes' rays still has a place
+        // if all of them turn out doubtful.
+        __shared__ uint32_t doubt_smem[kBlock / 32][kDoubtList];
+        uint32_t* const doubt = doubt_smem[threadIdx.x >> 5];
         uint32_t doubts = 0;
         while (true) {
             const uint32_t leafm = __ballot_sync(kFull, st.cur < 0);
             const uint32_t nodem = __ballot_sync(kFull, st.stepping());
-            bool take = more && (!AnyHit || doubts < kDoubtStop);
+            bool take = more && doubts < kDoubtStop;
             if ((leafm | nodem) == 0 || (take && uint32_t(__popc(leafm | nodem)) <= refill)) {
                 const bool idle = st.cur >= kDone;
-                const bool doubtful = AnyHit && st.cur == kDone && st.doubtful;
+                bool doubtful = false;
                 if (st.cur == kDone) {
-                    if (!doubtful) done(i, st.key != kNoIndex);
+                    if (st.tri != kNoIndex)
+                        doubtful = !in_own_box(tris, st.tri, r, qinv, tmin, AnyHit ? st.t : st.tl);
+                    if (!doubtful) done(i, st.tri != kNoIndex);
                     st.cur = kFree;
                 }
-                if constexpr (AnyHit) {
-                    const uint32_t m = __ballot_sync(kFull, doubtful);
-                    if (doubtful) doubt[doubts + __popc(m & ((1u << lane_id()) - 1u))] = i;
-                    doubts += __popc(m);
-                    take = more && doubts < kDoubtStop;
-                }
+                const uint32_t m = __ballot_sync(kFull, doubtful);
+                if (doubtful) doubt[doubts + __popc(m & ((1u << lane_id()) - 1u))] = i;
+                doubts += __popc(m);
+                take = more && doubts < kDoubtStop;
                 if (!take) {
                     if ((leafm | nodem) == 0) break;
                     continue;   // the busy lanes go on
@@ -250,6 +251,7 @@ __device__ __forceinline__ void traverse_queue(const DevScene& s, const DevScene
                         if constexpr (Multi) {
                             nodes = Tree == 4 ? table[sid].qnodes4 : table[sid].qnodes;
                             tris = table[sid].tris;
+                            qinv = table[sid].qinv;
                             r = make_quant_ray(table[sid], o, d);
                         } else {
                             r = make_quant_ray(s, o, d);
@@ -273,24 +275,24 @@ __device__ __forceinline__ void traverse_queue(const DevScene& s, const DevScene
                     }
             }
         }
-        if constexpr (AnyHit) {
-            auto trace_one = [&](uint32_t e) {
-                float3 o, d;
-                float tmax;
-                const uint32_t sid = load(e, o, d, tmax);
-                const DevScene& es = Multi ? table[sid] : s;
-                HitRec h;
-                done(e, trace<true, Count>(es, make_ray(o, d), tmin, tmax, h, &tw));
-            };
-            __syncwarp();
-            for (uint32_t k = lane_id(); k < doubts; k += 32u) trace_one(doubt[k]);
-            while (more) {
-                uint32_t base = 0;
-                if (lane_id() == 0) base = atomicAdd(cursor, 32u);
-                base = __shfl_sync(kFull, base, 0);
-                more = base < count;
-                if (base + lane_id() < count) trace_one(base + lane_id());
-            }
+        auto trace_one = [&](uint32_t e) {
+            float3 o, d;
+            float tmax;
+            const uint32_t sid = load(e, o, d, tmax);
+            const DevScene& es = Multi ? table[sid] : s;
+            HitRec h;
+            const bool found = trace<AnyHit, Count>(es, make_ray(o, d), tmin, tmax, h, &tw);
+            if (!AnyHit && found) hit(e, h.u, h.v, __uint_as_float(h.inst), __uint_as_float(h.prim));
+            done(e, found);
+        };
+        __syncwarp();
+        for (uint32_t k = lane_id(); k < doubts; k += 32u) trace_one(doubt[k]);
+        while (more) {
+            uint32_t base = 0;
+            if (lane_id() == 0) base = atomicAdd(cursor, 32u);
+            base = __shfl_sync(kFull, base, 0);
+            more = base < count;
+            if (base + lane_id() < count) trace_one(base + lane_id());
         }
     }
     if (Count) flush_work(tw, work_out);

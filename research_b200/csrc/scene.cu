@@ -288,6 +288,7 @@ rr_status rr_scene_create(rr_ctx* ctx, const rr_scene_desc* d, rr_scene** out) {
         RR_UP(bvh.qnodes4.data(), bvh.qnodes4.size() * sizeof(uint4), qnodes4, const uint4*);
         s->dev.qbase = make_float3(bvh.qbase[0], bvh.qbase[1], bvh.qbase[2]);
         s->dev.qscale = make_float3(bvh.qscale[0], bvh.qscale[1], bvh.qscale[2]);
+        s->dev.qinv = make_float3(1.0f / bvh.qscale[0], 1.0f / bvh.qscale[1], 1.0f / bvh.qscale[2]);
     }
     RR_UP(trirec.data(), trirec.size() * sizeof(float4), tris, const float4*);
     RR_UP(d->vertices, size_t(d->vertex_count) * sizeof(GpuVertex), vertices, const float4*);

@@ -1,8 +1,10 @@
-"""GPU tests of any-hit rays that meet a surface within a rounding of their
-far bound, in scenes where most shadow rays do: the queue traversal lists
-them per warp and traces them in the full-precision tree. The tolerance is
-zero: the queues' images are those of variant 7, which walks that tree alone,
-and the reuse passes' are those of their per-pixel form, which keeps no list."""
+"""GPU tests of rays whose hits the quantized boxes do not decide, in scenes
+where many are: any-hit rays that meet a surface within a rounding of their
+far bound, and rays that leave triangles so large that the triangle test's
+rounding reaches the near bound. The queue traversal lists them per warp and
+traces them in the full-precision tree. The tolerance is zero: the queues'
+images are those of variant 7, which walks that tree alone, and the reuse
+passes' are those of their per-pixel form, which keeps no list."""
 import ctypes as C
 
 import numpy as np
@@ -11,9 +13,9 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def floor_and_ceiling(rr, height, light_y, intensity, tess=16):
+def floor_and_ceiling(rr, height, light_y, intensity, tess=16, emissive=0.0):
     """Two tessellated squares, `height` apart and as wide each way, lit by a
-    point light at light_y."""
+    point light at light_y, or by the ceiling's own emission."""
     g = np.linspace(-height, height, tess + 1, dtype=np.float32)
     x, z = np.meshgrid(g, g, indexing="ij")
     n = (tess + 1) ** 2
@@ -33,22 +35,27 @@ def floor_and_ceiling(rr, height, light_y, intensity, tess=16):
     mt = np.zeros(2, rr.MATERIAL)
     mt["base_color"][:] = 0.8
     mt["roughness"] = 1.0
+    mt["emissive"][1] = emissive
     inst = np.zeros(2, rr.INSTANCE)
     inst["transform"] = np.eye(4, dtype=np.float32).reshape(-1)
     inst["mesh_index"] = [0, 1]
-    lights = np.zeros(1, rr.LIGHT)
-    lights["position"] = [0.013 * height, light_y, -0.021 * height]
-    lights["emission"] = 1.0
-    lights["intensity"] = intensity
+    lights = np.zeros(0 if emissive else 1, rr.LIGHT)
+    if not emissive:
+        lights["position"] = [0.013 * height, light_y, -0.021 * height]
+        lights["emission"] = 1.0
+        lights["intensity"] = intensity
     return {"vertices": v, "indices": idx, "meshes": m, "materials": mt, "instances": inst, "lights": lights}
 
 
 # A light 0.01 behind a ceiling 300 up: shadow rays end 0.01 before a light,
 # at the ceiling. And a ceiling so far away that 0.01 is lost in the distance,
-# with a light on it.
+# with a light on it, or emitting itself (the floor's triangles are 4e4 wide:
+# three in a hundred of the rays that leave it hit it again at 1e-3, if
+# nothing but their grown boxes keeps them from it).
 SCENES = {
     "behind": lambda rr: floor_and_ceiling(rr, 300.0, np.float32(300.01), 1e5),
     "on": lambda rr: floor_and_ceiling(rr, 3e5, 3e5, 1e11),
+    "emitting": lambda rr: floor_and_ceiling(rr, 3e5, 0.0, 0.0, emissive=5.0),
 }
 
 
@@ -62,34 +69,36 @@ def _height(name):
 
 @pytest.mark.parametrize("name", list(SCENES))
 def test_shadow_rays_at_their_bound(rr, ctx, torch_cuda, name):
-    """Some 160 rays for each resident warp: lists fill, and the rest of the
-    queue goes to the loop after them."""
+    """Some 160 shadow rays for each resident warp, and 1100 shadow and second
+    extension rays in the emitting scene: lists fill, and the rest of the queue
+    goes to the loop after them."""
     torch = torch_cuda
     L = rr.lib()
     st = torch.cuda.current_stream().cuda_stream
     scene = rr.Scene(ctx, SCENES[name](rr))
-    W, H, spp = 511, 385, 4
+    W, H = 511, 385
+    bounces, spp, mode = (2, 28, rr.PT_FLAG_EMITTERS) if name == "emitting" else (1, 4, 0)
     cam = _view(rr, _height(name), W, H)
-    images = {}
+
+    def render(variant, flags):
+        ctx.check(L.rr_pathtracer_set_variants(ctx.handle, variant, variant))
+        out = torch.empty((spp, H, W, 4), device="cuda")
+        p = rr.PtParams(3, bounces, spp, flags | mode)
+        ctx.check(L.rr_pathtracer_execute(ctx.handle, scene.handle, C.byref(cam), C.byref(p), out.data_ptr(), st))
+        return out
+
     try:
+        ref = render(7, 0)
+        if name != "behind":
+            lit = int((ref[..., :3].amax(-1) > 0).sum())
+            assert 0 < lit < ref[..., 0].numel()
         for v in range(rr.PT_VARIANT_COUNT):
             for flags in (0, rr.PT_FLAG_COUNT_TRAVERSAL):
-                ctx.check(L.rr_pathtracer_set_variants(ctx.handle, v, v))
-                out = torch.empty((spp, H, W, 4), device="cuda")
-                p = rr.PtParams(3, 1, spp, flags)
-                ctx.check(L.rr_pathtracer_execute(ctx.handle, scene.handle, C.byref(cam), C.byref(p), out.data_ptr(),
-                                                  st))
-                images[v, flags] = out.cpu().numpy()
+                bad = int((render(v, flags).view(torch.int32) != ref.view(torch.int32)).any(-1).sum())
+                assert bad == 0, f"variant {v}, flags {flags}: {bad} paths differ"
     finally:
         ctx.check(L.rr_pathtracer_set_variants(ctx.handle, 4, 4))
         scene.close()
-    ref = images[7, 0]
-    if name != "behind":
-        lit = ref[..., :3].max(-1) > 0
-        assert 0 < lit.sum() < lit.size
-    for (v, flags), got in images.items():
-        bad = int((got.view(np.uint32) != ref.view(np.uint32)).any(-1).sum())
-        assert bad == 0, f"variant {v}, flags {flags}: {bad} paths differ"
 
 
 def test_batch_shadow_rays_at_their_bound(rr, ctx, torch_cuda):
