@@ -165,13 +165,13 @@ constexpr int kWtRows = kTileH + 2, kWtElems = kHaloW * kWtRows;   // elements t
 constexpr uint32_t kTileBoxBytes = uint32_t(kTileElems * 16);      // one image's box of a TMA-staged tile
 
 struct TileSmem {
-    float4 rad[kTileElems];        // (r, g, b, 1); zero for a G-buffer miss
+    float4 rad[kTileElems];        // (r, g, b, 1); all zero for a G-buffer miss
     float p[7][kTileElems];        // position, unit normal, luminance
     float wt[kPairFwd][kWtElems];
 };
 constexpr uint32_t kTileSmem = sizeof(TileSmem);
-// staged: the three boxes as they are copied (the first over rad's place:
-// it is converted in place), and an mbarrier
+// staged: behind the tile, from a multiple of 128 bytes on, the three boxes
+// as they are copied, and an mbarrier
 constexpr uint32_t kTileSmemTma = kTileSmem + 3 * kTileBoxBytes + 128;
 
 RR_D float max_nan(float a, float b) {
@@ -374,9 +374,11 @@ __global__ void __launch_bounds__(kTileThreads, 2) atrous_tile_kernel(
             p = __ldg(gpos + k);
             n = __ldg(nrm + k);
         }
-        // A miss: no weight (it is infinitely far from every surface), no radiance.
+        // A miss: no weight (it is infinitely far from every surface; where
+        // sigma_position^2 is infinite too that makes a NaN, which the sum
+        // below replaces), no radiance.
         const bool miss = p.w < 0.0f;
-        t.rad[e] = miss ? make_float4(0.0f, 0.0f, 0.0f, 1.0f) : make_float4(r.x, r.y, r.z, 1.0f);
+        t.rad[e] = miss ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : make_float4(r.x, r.y, r.z, 1.0f);
         t.p[0][e] = miss ? INFINITY : p.x;
         t.p[1][e] = miss ? INFINITY : p.y;
         t.p[2][e] = miss ? INFINITY : p.z;
@@ -440,9 +442,10 @@ __global__ void __launch_bounds__(kTileThreads, 2) atrous_tile_kernel(
         #pragma unroll
         for (int tx = -2; tx <= 2; ++tx) {
             const int e = ce + ty * kHaloW + tx;
-            const float w = tx == 0 && ty == 0 ? wc
-                            : pair_forward(tx, ty) ? t.wt[pair_index(tx, ty)][ce] : t.wt[pair_index(-tx, -ty)][e];
+            float w = tx == 0 && ty == 0 ? wc
+                      : pair_forward(tx, ty) ? t.wt[pair_index(tx, ty)][ce] : t.wt[pair_index(-tx, -ty)][e];
             const ulonglong2 r = *reinterpret_cast<const ulonglong2*>(&t.rad[e]);
+            if (!FastDiv && hi2(r.y) == 0.0f) w = 0.0f;   // a miss
             frg = add2(frg, mul2(r.x, both(w)));
             fbw = add2(fbw, mul2(r.y, both(w)));
         }
