@@ -311,7 +311,8 @@ RR_D bool trace_step(const DevScene& s, const Ray& r, float tmin, HitRec& hit, T
 
 // One node of the 4-wide tree (8 float4 per node: lo.x, hi.x, lo.y, hi.y,
 // lo.z, hi.z of children 0..3, their references and their triangle counts;
-// unused slots hold a point box at 1e30, never reached). The four child
+// unused slots hold a point box at 1e30, which only a ray that is not a number
+// meets, and reference 0, the root, which is nobody's child). The four child
 // boxes are tested with box_pair's arithmetic, hit leaf children are
 // intersected right away, and the hit inner children are visited in
 // distance order (closest hit nearest first, any hit farthest first, ties
@@ -362,7 +363,7 @@ RR_D bool trace_step4(const DevScene& s, const Ray& r, float tmin, HitRec& hit, 
     int m = 0;
     #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const bool in = h[k] && R[k] >= 0 && nr[k] <= hit.t;
+        const bool in = h[k] && R[k] > 0 && nr[k] <= hit.t;
         m += in ? 1 : 0;
         key[k] = in ? (AnyHit ? -nr[k] : nr[k]) : INFINITY;
         nd[k] = R[k];
