@@ -480,9 +480,13 @@ using BatchShadowKernel = void (*)(const DevScene*, float4* const*, const float4
 // traced by kVariantFull's kernel whatever the variant. kVariantDefault is
 // the fastest on the 1M-triangle room (extension / shadow rays of the 1080p
 // frame 8.9 / 5.2 ms; 9.1 / 5.2 with the whole stack in local memory,
-// binary tree 9.9 / 6.0).
+// binary tree 9.9 / 6.0). kVariantFull's form differs for the two kinds of
+// rays: on the same room with one mesh 1e7 away (not quantized), extension rays
+// with 4 blocks per SM and 8 stack entries in shared memory, shadow rays
+// with 5 blocks and a local stack: 16.2 / 11.0 ms, 16.6 / 11.8 both with 4 blocks and
+// a local stack.
 constexpr int kVariantFull = 7, kVariantDefault = 4;
-#define RR_TRAVERSAL_VARIANTS(kernel, v)                   \
+#define RR_TRAVERSAL_VARIANTS(kernel, v, full_blocks, full_smem) \
     switch (v) {                                           \
     case 0: return kernel<Count, 4, 2, 8>;                 \
     case 1: return kernel<Count, 5, 2, 0>;                 \
@@ -490,23 +494,23 @@ constexpr int kVariantFull = 7, kVariantDefault = 4;
     case 3: return kernel<Count, 4, 4, 0>;                 \
     case 5: return kernel<Count, 5, 2, 12>;                \
     case 6: return kernel<Count, 5, 4, 8>;                 \
-    case kVariantFull: return kernel<Count, 4, 0, 0>;      \
+    case kVariantFull: return kernel<Count, full_blocks, 0, full_smem>; \
     default: return kernel<Count, 4, 4, 12>;               \
     }
 
 template <bool Count>
-BatchQueueKernel extend_batch_variant(int v) { RR_TRAVERSAL_VARIANTS(extend_batch_kernel, v) }
+BatchQueueKernel extend_batch_variant(int v) { RR_TRAVERSAL_VARIANTS(extend_batch_kernel, v, 4, 8) }
 template <bool Count>
-BatchShadowKernel shadow_batch_variant(int v) { RR_TRAVERSAL_VARIANTS(shadow_batch_kernel, v) }
+BatchShadowKernel shadow_batch_variant(int v) { RR_TRAVERSAL_VARIANTS(shadow_batch_kernel, v, 5, 0) }
 
 using QueueKernel = void (*)(DevScene, const float4*, const float4*, float4*, const uint32_t*, uint32_t*,
                              unsigned long long*, uint32_t);
 using ShadowKernel = void (*)(DevScene, const float4*, const float4*, const float4*, float4*, const uint32_t*,
                               uint32_t*, unsigned long long*);
 template <bool Count>
-QueueKernel extend_variant(int v) { RR_TRAVERSAL_VARIANTS(extend_kernel, v) }
+QueueKernel extend_variant(int v) { RR_TRAVERSAL_VARIANTS(extend_kernel, v, 4, 8) }
 template <bool Count>
-ShadowKernel shadow_variant(int v) { RR_TRAVERSAL_VARIANTS(shadow_kernel, v) }
+ShadowKernel shadow_variant(int v) { RR_TRAVERSAL_VARIANTS(shadow_kernel, v, 5, 0) }
 
 // When a bounce's extension rays are refilled (traverse_queue).
 uint32_t refill_of(uint32_t bounce) { return bounce == 0 ? 0u : kBusyLanes; }
