@@ -170,7 +170,10 @@ rr_status rr_pathtracer_set_overlap(rr_ctx* ctx, int enable);
 
 /* Autotuner: renders the given frame once per variant with stage timing,
  * keeps the fastest extension and shadow variants on this context and
- * reports every measured time (ms per frame). Synchronises the device. */
+ * reports every measured time (ms per frame). A scene that runs one kernel
+ * whatever the variant (see above) is timed once: the context keeps the
+ * variants it has, and they are reported as the best. Synchronises the
+ * device. */
 typedef struct rr_pt_tune_result {
     double extend_ms[RR_PT_VARIANT_COUNT];
     double shadow_ms[RR_PT_VARIANT_COUNT];
@@ -222,7 +225,8 @@ rr_status rr_batch_execute(rr_ctx* ctx, rr_batch* batch, const GpuCameraData* ca
                            const rr_pt_params* params, float* const* radiance_out, void* stream);
 
 /* rr_pathtracer_tune for a batch: times every traversal variant on the
- * batch, keeps the fastest on the context (graphs are recaptured), then
+ * batch, keeps the fastest on the context (graphs are recaptured; once, and
+ * the context's own, where a scene of the batch has one kernel only), then
  * times the batch's two forms with those variants and keeps the faster on
  * the batch (rr_batch_get_mode). */
 rr_status rr_batch_tune(rr_ctx* ctx, rr_batch* batch, const GpuCameraData* cameras,

@@ -512,8 +512,15 @@ extern "C" rr_status rr_pathtracer_tune(rr_ctx* ctx, const rr_scene* scene, cons
     rr_pt_params q = *p;
     q.flags = RR_PT_FLAG_TIME_STAGES;
     double best_e = 1e30, best_s = 1e30;
+    const int kept_e = ctx->extend_variant, kept_s = ctx->shadow_variant;
+    const bool choice = scene->dev.qnodes4 != nullptr;   // otherwise every variant runs one kernel
     out->best_extend = out->best_shadow = 0;
     for (int v = 0; v < RR_PT_VARIANT_COUNT; ++v) {
+        if (!choice && v > 0) {
+            out->extend_ms[v] = out->extend_ms[0];
+            out->shadow_ms[v] = out->shadow_ms[0];
+            continue;
+        }
         ctx->extend_variant = v;
         ctx->shadow_variant = v;
         // one untimed pass to settle caches and clocks, then one timed pass
@@ -527,6 +534,7 @@ extern "C" rr_status rr_pathtracer_tune(rr_ctx* ctx, const rr_scene* scene, cons
         if (st.ms_extend < best_e) { best_e = st.ms_extend; out->best_extend = v; }
         if (st.ms_shadow < best_s) { best_s = st.ms_shadow; out->best_shadow = v; }
     }
+    if (!choice) { out->best_extend = kept_e; out->best_shadow = kept_s; }
     ctx->extend_variant = out->best_extend;
     ctx->shadow_variant = out->best_shadow;
     return RR_OK;
@@ -779,10 +787,17 @@ extern "C" rr_status rr_batch_tune(rr_ctx* ctx, rr_batch* B, const GpuCameraData
     rr_status s;
     if ((s = rr_pathtracer_stats(ctx, &st, 1)) != RR_OK) return s;
     double best_e = 1e300, best_s = 1e300;
+    const int kept_e = ctx->extend_variant, kept_s = ctx->shadow_variant;
+    const bool choice = B->quantized;   // as in rr_pathtracer_tune
     rr_pt_params warm = *p, q = *p;
     warm.flags = 0;
     q.flags = RR_PT_FLAG_TIME_STAGES;
     for (int v = 0; v < RR_PT_VARIANT_COUNT; ++v) {
+        if (!choice && v > 0) {
+            out->extend_ms[v] = out->extend_ms[0];
+            out->shadow_ms[v] = out->shadow_ms[0];
+            continue;
+        }
         ctx->extend_variant = v;
         ctx->shadow_variant = v;
         if ((s = rr_batch_execute(ctx, B, cams, &warm, radiance_out, stream)) != RR_OK) return s;
@@ -793,6 +808,7 @@ extern "C" rr_status rr_batch_tune(rr_ctx* ctx, rr_batch* B, const GpuCameraData
         if (st.ms_extend < best_e) { best_e = st.ms_extend; out->best_extend = v; }
         if (st.ms_shadow < best_s) { best_s = st.ms_shadow; out->best_shadow = v; }
     }
+    if (!choice) { out->best_extend = kept_e; out->best_shadow = kept_s; }
     ctx->extend_variant = out->best_extend;
     ctx->shadow_variant = out->best_shadow;
     // the batch's form: each timed (after one warm-up call) with the caller's

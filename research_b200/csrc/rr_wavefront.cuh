@@ -481,10 +481,10 @@ using BatchShadowKernel = void (*)(const DevScene*, float4* const*, const float4
 // the fastest on the 1M-triangle room (extension / shadow rays of the 1080p
 // frame 8.9 / 5.2 ms; 9.1 / 5.2 with the whole stack in local memory,
 // binary tree 9.9 / 6.0). kVariantFull's form differs for the two kinds of
-// rays: on the same room with one mesh 1e7 away (not quantized), extension rays
-// with 4 blocks per SM and 8 stack entries in shared memory, shadow rays
-// with 5 blocks and a local stack: 16.2 / 11.0 ms, 16.6 / 11.8 both with 4 blocks and
-// a local stack.
+// rays: on the same room with one mesh 1e7 away (not quantized) 16.2 / 11.0 ms
+// with 4 blocks per SM and 8 stack entries in shared memory for extension
+// rays, 5 blocks and a local stack for shadow rays; 16.6 / 11.8 with 4 blocks
+// and a local stack for both.
 constexpr int kVariantFull = 7, kVariantDefault = 4;
 #define RR_TRAVERSAL_VARIANTS(kernel, v, full_blocks, full_smem) \
     switch (v) {                                           \
