@@ -155,6 +155,7 @@ rr_status rr_pathtracer_stats(rr_ctx* ctx, rr_pt_stats* out, int reset_times);
  *      use it whatever the variant.
  * Results are identical for every variant; only speed differs. */
 #define RR_PT_VARIANT_COUNT 8
+#define RR_PT_VARIANT_DEFAULT 4
 rr_status rr_pathtracer_set_variants(rr_ctx* ctx, int extend_variant, int shadow_variant);
 
 /* Shadow overlap (default on): the path tracers (rr_pathtracer_execute,

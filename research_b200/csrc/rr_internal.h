@@ -47,8 +47,8 @@ struct rr_ctx {
     uint32_t* counters = nullptr;          // kCounterWords
     unsigned long long* work64 = nullptr;  // traversal work: ext nodes, ext tris, shadow nodes, shadow tris
     uint32_t last_max_bounces = 0;
-    int extend_variant = 4;                // traversal variants (rr_pathtracer_set_variants); 4: kVariantDefault
-    int shadow_variant = 4;
+    int extend_variant = RR_PT_VARIANT_DEFAULT;   // rr_pathtracer_set_variants
+    int shadow_variant = RR_PT_VARIANT_DEFAULT;
     bool last_counted = false;
     uint64_t launches = 0;                 // kernels issued by this context
     double stage_ms[4] = {0, 0, 0, 0};     // raygen, extend, shade, shadow

@@ -477,15 +477,15 @@ using BatchShadowKernel = void (*)(const DevScene*, float4* const*, const float4
                                    const uint32_t*, uint32_t*, unsigned long long*);
 // Traversal kernel variants (rr_pathtracer_set_variants): MinBlocks x tree x
 // stack entries in shared memory. A scene whose trees are not quantized is
-// traced by kVariantFull's kernel whatever the variant. kVariantDefault is
-// the fastest on the 1M-triangle room (extension / shadow rays of the 1080p
+// traced by kVariantFull's kernel whatever the variant. RR_PT_VARIANT_DEFAULT
+// (4) is the fastest on the 1M-triangle room (extension / shadow rays of the 1080p
 // frame 8.9 / 5.2 ms; 9.1 / 5.2 with the whole stack in local memory,
 // binary tree 9.9 / 6.0). kVariantFull's form differs for the two kinds of
 // rays: on the same room with one mesh 1e7 away (not quantized) 16.2 / 11.0 ms
 // with 4 blocks per SM and 8 stack entries in shared memory for extension
 // rays, 5 blocks and a local stack for shadow rays; 16.6 / 11.8 with 4 blocks
 // and a local stack for both.
-constexpr int kVariantFull = 7, kVariantDefault = 4;
+constexpr int kVariantFull = 7;
 #define RR_TRAVERSAL_VARIANTS(kernel, v, full_blocks, full_smem) \
     switch (v) {                                           \
     case 0: return kernel<Count, 4, 2, 8>;                 \

@@ -70,6 +70,7 @@ PT_FLAG_TIME_STAGES = 2
 PT_FLAG_GRAPH = 4
 PT_FLAG_EMITTERS = 8
 PT_VARIANT_COUNT = 8
+PT_VARIANT_DEFAULT = 4
 TRACE_ANY_HIT, TRACE_WIDE = 1, 2   # rr_trace_counted flags
 BATCH_WAVEFRONT = 0
 BATCH_PER_SCENE = 1

@@ -52,5 +52,17 @@ def ctx(rr, torch_cuda):
     c.close()
 
 
+@pytest.fixture(autouse=True)
+def default_traversal(request):
+    """The shared context walks the library's default tree in every test that
+    does not choose another one itself."""
+    c = request.getfixturevalue("ctx") if "ctx" in request.fixturenames else None
+    yield
+    if c is not None:
+        rr = request.getfixturevalue("rr")
+        d = rr.PT_VARIANT_DEFAULT
+        c.check(rr.lib().rr_pathtracer_set_variants(c.handle, d, d))
+
+
 def to_np(t):
     return t.detach().cpu().numpy()
