@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstring>
 #include <future>
+#include <thread>
 
 namespace rr {
 namespace {
@@ -202,6 +203,26 @@ bool quant_ref(int32_t ref, int32_t count, uint32_t& out) {
     return true;
 }
 
+// f(first, end, chunk) over [0, n) in chunks of kChunk on the machine's threads; the
+// chunks do not depend on how many there are. False as soon as a chunk says so.
+constexpr size_t kChunk = 16384;
+template <class F>
+bool for_chunks(size_t n, F f) {
+    const size_t chunks = (n + kChunk - 1) / kChunk;
+    std::atomic<size_t> next{0};
+    std::atomic<bool> ok{true};
+    auto work = [&] {
+        for (size_t c = next++; c < chunks && ok; c = next++)
+            if (!f(c * kChunk, std::min(n, (c + 1) * kChunk), c)) ok = false;
+    };
+    const size_t threads = std::min<size_t>({chunks, std::thread::hardware_concurrency(), 16});
+    std::vector<std::future<void>> others;
+    for (size_t t = 1; t < threads; ++t) others.push_back(std::async(std::launch::async, work));
+    work();
+    for (auto& o : others) o.get();
+    return ok;
+}
+
 // The quantized forms of both trees: every box plane goes outwards to a plane
 // of a 15-bit grid over the scene's bounds, so a box only grows. Refused (the
 // traversals then read the trees in full precision) where the boxes would
@@ -250,9 +271,14 @@ bool quantize_trees(BvhBuild& out) {
         return true;
     };
     auto area = [](const double* e) { return e[0] * e[1] + e[1] * e[2] + e[2] * e[0]; };
-    double full = 0.0, grown = 0.0;
+    // One million triangles: 220 ms on one thread, 70 on eight. With the 4-wide
+    // layout beside the binary one a build takes 1.50 s; 1.64 before there were
+    // quantized trees, 1.84 with everything one after the other.
+    std::vector<double> full((n + kChunk - 1) / kChunk, 0.0), grown(full.size(), 0.0);
     out.qnodes.resize(n * 2);
-    for (size_t g = 0; g < n; ++g) {
+    const bool fits = for_chunks(n, [&](size_t first_node, size_t end, size_t chunk) {
+      double f = 0.0, q = 0.0;
+      for (size_t g = first_node; g < end; ++g) {
         const float4& d = out.nodes[g * 4 + 3];
         int32_t ref[2], cnt[2];
         std::memcpy(ref, &d.x, 8);
@@ -266,15 +292,26 @@ bool quantize_trees(BvhBuild& out) {
                 if (!pack(a, l, h, w[a], eq[a])) return false;
                 e[a] = double(h) - double(l);
             }
-            full += area(e);
-            grown += area(eq);
+            f += area(e);
+            q += area(eq);
             if (!quant_ref(ref[c], cnt[c], r)) return false;
             out.qnodes[g * 2 + c] = make_uint4(w[0], w[1], w[2], r);
         }
+      }
+      full[chunk] = f;
+      grown[chunk] = q;
+      return true;
+    });
+    if (!fits) return false;
+    double sum_full = 0.0, sum_grown = 0.0;
+    for (size_t c = 0; c < full.size(); ++c) {
+        sum_full += full[c];
+        sum_grown += grown[c];
     }
-    if (!(grown <= kQuantGrowth * full)) return false;
+    if (!(sum_grown <= kQuantGrowth * sum_full)) return false;
     out.qnodes4.resize(n4 * 4);
-    for (size_t g = 0; g < n4; ++g) {
+    return for_chunks(n4, [&](size_t first_node, size_t end, size_t) {
+      for (size_t g = first_node; g < end; ++g) {
         const float* f = &out.nodes4[g * 8].x;
         for (int k = 0; k < 4; ++k) {
             uint32_t w[3], r;
@@ -291,8 +328,9 @@ bool quantize_trees(BvhBuild& out) {
             if (!quant_ref(ref, cnt, r)) return false;
             out.qnodes4[g * 4 + k] = make_uint4(w[0], w[1], w[2], r);
         }
-    }
-    return true;
+      }
+      return true;
+    });
 }
 
 } // namespace
@@ -317,12 +355,13 @@ BvhBuild build_bvh(const std::vector<float>& tri_world, int /*threads*/) {
     if (n > 0) B.build(0, 0, n, 0);
     else nodes[0].box = Box();
     out.max_depth = B.depth_max.load() + 1;
-    {
+    // the 4-wide layout, beside the binary one below (a small scene's after it)
+    std::future<void> wide = std::async(n > 50000 ? std::launch::async : std::launch::deferred, [&] {
         Wide4 W{nodes, out.nodes4};
         if (n > 0 && nodes[0].left >= 0) W.emit(W.frontier(0));
         else if (n > 0) W.emit(std::vector<uint32_t>{0u});   // the root is a leaf
         else W.emit(std::vector<uint32_t>{});
-    }
+    });
 
     // GPU layout: one GPU node per inner binary node, depth-first, left first.
     auto child_ref = [&](const Node& c, std::vector<int32_t>& gidx, int32_t ci, int32_t& ref, int32_t& cnt) {
@@ -342,6 +381,7 @@ BvhBuild build_bvh(const std::vector<float>& tri_world, int /*threads*/) {
         out.nodes.push_back(mk4(lo0, hi0, lo1, hi1));
         out.nodes.push_back(mk4(lo2, hi2, lo2, hi2));
         out.nodes.push_back(mk4(i2f(~int32_t(0)), i2f(~int32_t(0)), i2f(int32_t(r.count)), i2f(0)));
+        wide.get();
         if (!quantize_trees(out)) { out.qnodes.clear(); out.qnodes4.clear(); }
         return out;
     }
@@ -368,6 +408,7 @@ BvhBuild build_bvh(const std::vector<float>& tri_world, int /*threads*/) {
         out.nodes[g * 4 + 2] = mk4(c0.box.lo[2], c0.box.hi[2], c1.box.lo[2], c1.box.hi[2]);
         out.nodes[g * 4 + 3] = mk4(i2f(r0), i2f(r1), i2f(k0), i2f(k1));
     }
+    wide.get();
     if (!quantize_trees(out)) { out.qnodes.clear(); out.qnodes4.clear(); }
     return out;
 }
