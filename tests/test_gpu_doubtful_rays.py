@@ -157,3 +157,30 @@ def test_reuse_shadow_rays_at_their_bound(rr, ctx, torch_cuda, reuse):
     assert got[0][-1].reshape(-1, 4)[:, 0].any()
     for k, (a, b) in enumerate(zip(*got)):
         np.testing.assert_array_equal(a, b, err_msg=f"image {k}")
+
+
+def test_inline_rays_that_leave_large_triangles(rr, ctx, torch_cuda):
+    """ReSTIR DI's camera rays (traced in lanes) from just above the floor up
+    to the far ceiling: the same hits as in the scene with one instance more,
+    so far away that its trees are not quantized."""
+    torch = torch_cuda
+    L = rr.lib()
+    st = torch.cuda.current_stream().cuda_stream
+    W, H, height = 300, 200, 3e5
+    eye = (-0.943 * height, 1e-4, -0.4416 * height)
+    cam = rr.camera_data(rr.camera_desc(W, H, eye=eye, center=(-0.6 * height, height, -0.3 * height)))
+    arrays = SCENES["on"](rr)
+    far = arrays["instances"][:1].copy()
+    far[0]["transform"].reshape(4, 4)[:3, 3] += np.float32(1e13)
+    got = []
+    for a in (arrays, {**arrays, "instances": np.concatenate([arrays["instances"], far])}):
+        scene = rr.Scene(ctx, a)
+        z = [torch.zeros((H, W, 4), device="cuda") for _ in range(5)]
+        p = rr.DIParams(1, 4, 0, 0, 4, 15, 20, 0)
+        ctx.check(L.rr_restir_di_execute(ctx.handle, scene.handle, C.byref(cam), C.byref(p),
+                                         *[t.data_ptr() for t in z], st))
+        got.append([t.cpu().numpy() for t in z[:2]])
+        scene.close()
+    assert (got[1][0][..., 3] > 1e4).mean() > 0.9
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a.view(np.uint32), b.view(np.uint32))
