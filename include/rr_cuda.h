@@ -144,16 +144,21 @@ rr_status rr_pathtracer_stats(rr_ctx* ctx, rr_pt_stats* out, int reset_times);
 /* Traversal kernel variants (no reference counterpart; the reference uses
  * hardware ray queries): variant = tree x stack x occupancy target (blocks
  * of 256 threads per SM). 0 to 6 walk the scene's trees with boxes quantized
- * to a 15-bit grid (a box only grows, so hits are the same), a warp's lanes
- * in step, idle lanes taking new rays:
+ * to a 15-bit grid (a box only grows; a hit that the boxes in full precision
+ * would not offer does not count), a warp's lanes in step, idle lanes taking
+ * new rays:
  *   0, 1, 2, 5: binary tree: bottom 8 stack entries in shared memory; local
  *      stack, 5 blocks; local stack; bottom 12 in shared memory, 5 blocks;
  *   3, 4, 6: 4-wide tree (rr_pathtracer_variant_width): local stack; bottom
- *      12 entries in shared memory (4, the default); bottom 8, 5 blocks;
+ *      12 entries in shared memory (4, RR_PT_VARIANT_DEFAULT); bottom 8, 5
+ *      blocks;
  *   7: binary tree in full precision, one thread per ray. Scenes whose boxes
  *      the grid would grow too much (a few triangles far from all others)
  *      use it whatever the variant.
- * Results are identical for every variant; only speed differs. */
+ * Results are the same bits for every variant, only speed differs, but for a
+ * tie: where two surfaces lie within 1e-5 of each other along a closest-hit
+ * ray (an edge that two triangles share), 0 to 6 keep the lowest (t, instance,
+ * primitive), which 7 may pass over (about one ray in 10^8). */
 #define RR_PT_VARIANT_COUNT 8
 #define RR_PT_VARIANT_DEFAULT 4
 rr_status rr_pathtracer_set_variants(rr_ctx* ctx, int extend_variant, int shadow_variant);

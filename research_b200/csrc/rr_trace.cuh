@@ -418,7 +418,7 @@ RR_D bool trace4(const DevScene& s, const Ray& r, float tmin, float tmax, HitRec
 // 4-wide node 64 bytes, two.
 //
 // What bounds it: instruction issue (68 % active on the 1M-triangle room's
-// first bounce) and the L1 data path (69 %, node sectors and stack), no
+// first bounce) and the L1 data path (64 %, node sectors and stack), no
 // longer divergence: 16 of 32 lanes per instruction against 8 with one
 // thread per ray running its leaves' triangle loops inline.
 RR_D void load32(const void* p, u64& a, u64& b, u64& c, u64& d) {

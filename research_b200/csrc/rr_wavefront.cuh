@@ -148,7 +148,8 @@ __device__ __forceinline__ void flush_work(const TraceWork& w, unsigned long lon
 // 8.8 / 8.1 / 7.8 ms; on the quantized binary tree 12.5 / 6.9 ms; leaves as
 // references and one, two, three node steps a vote 11.5 / 10.8 / 10.5 and
 // 6.4 / 6.1 / 5.8 ms; 4-wide, two steps, stack in shared memory 9.3 / 5.2 ms;
-// camera rays without refill 8.9 ms.
+// camera rays without refill 8.9 ms; with every hit tested against its
+// triangle's own box (in_own_box) 9.4 / 5.3 ms.
 //
 // Tree 0: the binary tree in full precision, one thread per ray (scenes that
 // the grid does not serve).
@@ -479,8 +480,8 @@ using BatchShadowKernel = void (*)(const DevScene*, float4* const*, const float4
 // stack entries in shared memory. A scene whose trees are not quantized is
 // traced by kVariantFull's kernel whatever the variant. RR_PT_VARIANT_DEFAULT
 // (4) is the fastest on the 1M-triangle room (extension / shadow rays of the 1080p
-// frame 8.9 / 5.2 ms; 9.1 / 5.2 with the whole stack in local memory,
-// binary tree 9.9 / 6.0). kVariantFull's form differs for the two kinds of
+// frame 9.4 / 5.3 ms; 9.7 / 5.4 with the whole stack in local memory,
+// binary tree 10.4 / 6.0). kVariantFull's form differs for the two kinds of
 // rays: on the same room with one mesh 1e7 away (not quantized) 16.2 / 11.0 ms
 // with 4 blocks per SM and 8 stack entries in shared memory for extension
 // rays, 5 blocks and a local stack for shadow rays; 16.6 / 11.8 with 4 blocks
