@@ -153,8 +153,8 @@ rr_status rr_pathtracer_stats(rr_ctx* ctx, rr_pt_stats* out, int reset_times);
  *      12 entries in shared memory (4, RR_PT_VARIANT_DEFAULT); bottom 8, 5
  *      blocks;
  *   7: binary tree in full precision, one thread per ray. Scenes whose boxes
- *      the grid would grow too much (a few triangles far from all others)
- *      use it whatever the variant.
+ *      the grid would grow too much (a few triangles far from all others, a
+ *      dense object on a wide ground) use it whatever the variant.
  * Results are the same bits for every variant, only speed differs, but for a
  * tie: where two surfaces lie within 1e-5 of each other along a closest-hit
  * ray (an edge that two triangles share), 0 to 6 keep the lowest (t, instance,

@@ -203,6 +203,53 @@ bool quant_ref(int32_t ref, int32_t count, uint32_t& out) {
     return true;
 }
 
+// The most that grown boxes cost a ray anywhere in the tree. A ray that enters
+// a node's box enters a child's with the probability of their areas' ratio, so
+// the tests below a node add up from the leaves; to these come the nodes above
+// it, which any ray that gets there has passed. Returned: the largest ratio, over
+// all nodes, of that sum with the grown boxes to that with the tight ones. (A
+// sum over the whole tree would not do: a small object on a wide ground has
+// next to none of the area, and all of the rays once the camera looks at it.)
+// areas: tight and grown area of both children of each node; depth-first, so a
+// child's index is larger than its parent's.
+double worst_cost_ratio(const std::vector<float4>& nodes, const std::vector<float4>& areas) {
+    const size_t n = nodes.size() / 4;
+    std::vector<float2> cost(n);      // tests below a node: tight, grown
+    std::vector<float2> own(n);       // its own box's area
+    std::vector<uint16_t> depth(n, 0);
+    auto kids = [&](size_t g, int32_t* ref, int32_t* cnt) {
+        std::memcpy(ref, &nodes[g * 4 + 3].x, 8);
+        std::memcpy(cnt, &nodes[g * 4 + 3].z, 8);
+    };
+    for (size_t g = 0; g < n; ++g) {
+        int32_t ref[2], cnt[2];
+        kids(g, ref, cnt);
+        const float4 a = areas[g];
+        if (g == 0) own[0] = make_float2(std::max(a.x, a.z), std::max(a.y, a.w));
+        for (int c = 0; c < 2; ++c)
+            if (ref[c] >= 0) {
+                depth[ref[c]] = uint16_t(depth[g] + 1);
+                own[ref[c]] = c ? make_float2(a.z, a.w) : make_float2(a.x, a.y);
+            }
+    }
+    double worst = 1.0;
+    for (size_t g = n; g-- > 0;) {
+        int32_t ref[2], cnt[2];
+        kids(g, ref, cnt);
+        const float4 a = areas[g];
+        float2 sum = make_float2(1.0f, 1.0f);
+        for (int c = 0; c < 2; ++c) {
+            const float2 below = ref[c] >= 0 ? cost[ref[c]] : make_float2(float(cnt[c]), float(cnt[c]));
+            const float t = c ? a.z : a.x, q = c ? a.w : a.y;
+            sum.x += (own[g].x > t ? t / own[g].x : 1.0f) * below.x;
+            sum.y += (own[g].y > q ? q / own[g].y : 1.0f) * below.y;
+        }
+        cost[g] = sum;
+        worst = std::max(worst, (double(depth[g]) + sum.y) / (double(depth[g]) + sum.x));
+    }
+    return worst;
+}
+
 // f(first, end, chunk) over [0, n) in chunks of kChunk on the machine's threads; the
 // chunks do not depend on how many there are. False as soon as a chunk says so.
 constexpr size_t kChunk = 16384;
@@ -233,7 +280,16 @@ bool for_chunks(size_t n, F f) {
 // against full precision (4.7 / 3.4): growth 1.003 2.6 / 1.6, 1.010 2.7 / 1.7,
 // 1.036 3.4 / 2.1, 1.094 5.3 / 3.5, 1.2 10.0 / 7.3. The 10M-triangle instanced
 // scenes grow by 1.006 and 1.008.
+// Also refused where some part of the tree costs too much (worst_cost_ratio):
+// the camera may look at just that. Path-traced 960 x 540 frames, 4 spp, both
+// kinds of rays, full precision over quantized time: the room (1.17) 1.9; 4096
+// instances in a box of 500 (1.56) 1.32, filled by its smallest instance 1.03
+// to 1.06; a sphere of 20,000 triangles on a ground 30, 60, 100, 150 times its
+// size (1.13, 1.25, 1.39, 1.85) 1.16, 1.10, 0.96, 0.92, and 3000 times 0.12; one
+// of 320,000 on a ground of 10, 20, 30, 60, 1000 times (1.36, 1.62, 1.88, 2.4,
+// 37) 1.25, 1.07, 1.02, 0.91, 0.085.
 constexpr double kQuantGrowth = 1.06;
+constexpr double kQuantWorst = 1.6;
 
 bool quantize_trees(BvhBuild& out) {
     const size_t n = out.nodes.size() / 4, n4 = out.nodes4.size() / 8;
@@ -271,10 +327,12 @@ bool quantize_trees(BvhBuild& out) {
         return true;
     };
     auto area = [](const double* e) { return e[0] * e[1] + e[1] * e[2] + e[2] * e[0]; };
-    // One million triangles: 220 ms on one thread, 70 on eight. With the 4-wide
-    // layout beside the binary one a build takes 1.50 s; 1.64 before there were
-    // quantized trees, 1.84 with everything one after the other.
+    // One million triangles: 220 ms on one thread, 70 on eight, and 60 for
+    // worst_cost_ratio. With the 4-wide layout beside the binary one a build
+    // takes 1.65 s; 1.78 before there were quantized trees, 1.98 with the
+    // quantization on one thread and one layout after the other.
     std::vector<double> full((n + kChunk - 1) / kChunk, 0.0), grown(full.size(), 0.0);
+    std::vector<float4> areas(n);
     out.qnodes.resize(n * 2);
     const bool fits = for_chunks(n, [&](size_t first_node, size_t end, size_t chunk) {
       double f = 0.0, q = 0.0;
@@ -292,8 +350,11 @@ bool quantize_trees(BvhBuild& out) {
                 if (!pack(a, l, h, w[a], eq[a])) return false;
                 e[a] = double(h) - double(l);
             }
-            f += area(e);
-            q += area(eq);
+            const double tight = area(e), large = area(eq);
+            f += tight;
+            q += large;
+            if (c == 0) { areas[g].x = float(tight); areas[g].y = float(large); }
+            else { areas[g].z = float(tight); areas[g].w = float(large); }
             if (!quant_ref(ref[c], cnt[c], r)) return false;
             out.qnodes[g * 2 + c] = make_uint4(w[0], w[1], w[2], r);
         }
@@ -309,6 +370,7 @@ bool quantize_trees(BvhBuild& out) {
         sum_grown += grown[c];
     }
     if (!(sum_grown <= kQuantGrowth * sum_full)) return false;
+    if (worst_cost_ratio(out.nodes, areas) > kQuantWorst) return false;
     out.qnodes4.resize(n4 * 4);
     return for_chunks(n4, [&](size_t first_node, size_t end, size_t) {
       for (size_t g = first_node; g < end; ++g) {
